@@ -275,6 +275,7 @@ def _declare(lib):
         sigs[f"clspmv_upload_{fmt}_f32"] = (I32, [S[fmt], S[fmt]])
         sigs[f"clspmv_device_free_{fmt}_f32"] = (I32, [S[fmt]])
     sigs.update({
+        "clspmv_device_trim": (I32, []),
         "clspmv_device_sort_coo_f32": (I32, [S["coo"], VP]),
         "clspmv_device_coo2csr_f32": (I32, [S["coo"], S["csr"], VP]),
         "clspmv_device_coo2dia_f32": (I32, [S["coo"], S["dia"], I32, VP]),

@@ -9,6 +9,11 @@ int cuda_status(cudaError_t e);
 // Counts `n` kernel launches and returns the status of the last launch.
 int after_launch(int n);
 
+// Device arrays that outlast a call, from the bounded list of released ones or cudaMalloc (device_pool.cu).
+// device_release waits for the device unless `idle` says that no work on the array is pending.
+int device_alloc(void** out, size_t bytes);
+void device_release(void* p, bool idle);
+
 // Format launchers (spmv_api.cu). With `atomic`, alpha*A*x is added into y
 // with red.global.add and beta is ignored (apply it first with
 // launch_prescale); several launches may then target one y concurrently.

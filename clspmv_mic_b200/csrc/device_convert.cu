@@ -11,7 +11,7 @@
 // clspmv_device_sort_coo_f32 sorts a device COO in place, stably, as
 // clspmv_sort_coo_f32 does on the host.
 //
-// Output arrays are cudaMalloc'ed and released with
+// Output arrays come from device_alloc and are released with
 // clspmv_device_free_<fmt> (an empty array still gets an allocation, so no
 // pointer is NULL after a success). Every call synchronises `stream`: sizes
 // are read back to size the outputs, once per call where the format allows.
@@ -63,27 +63,25 @@ int bits_for(long long n)   // bits of the largest value in [0, n)
 
 // Device arrays of one call on one stream, released at scope exit unless kept.
 struct Allocs {
+    cudaStream_t st;
     std::vector<void*> ptrs;
     int rc = CLSPMV_OK;
     bool keep = false;
-    explicit Allocs(cudaStream_t) {}
+    explicit Allocs(cudaStream_t s) : st(s) {}
     template <class T>
     T* get(size_t n)
     {
         if (rc) return nullptr;
         void* p = nullptr;
-        if (cudaMalloc(&p, std::max<size_t>(n, 1) * sizeof(T)) != cudaSuccess) {
-            cudaGetLastError();
-            rc = CLSPMV_ERR_ALLOC;
-            return nullptr;
-        }
+        if ((rc = clspmv::device_alloc(&p, std::max<size_t>(n, 1) * sizeof(T)))) return nullptr;
         ptrs.push_back(p);
         return static_cast<T*>(p);
     }
     ~Allocs()
     {
-        if (!keep)
-            for (void* p : ptrs) cudaFree(p);
+        if (keep || ptrs.empty()) return;
+        const bool idle = cudaStreamSynchronize(st) == cudaSuccess;   // the arrays were used on `st` alone
+        for (void* p : ptrs) clspmv::device_release(p, idle);
     }
 };
 
@@ -1555,7 +1553,7 @@ int clspmv_device_coo2bdia_f32(const clspmv_coo_f32* src, clspmv_bdia_f32* dst, 
         return rc;
     if ((rc = cuda_status(cudaMemcpy(bp, bptr.data(), sizeof(int) * bptr.size(), cudaMemcpyHostToDevice)))) return rc;
     O.keep = true;
-    cudaFree(dia.dia_offsets);   // the DIA data array becomes the BDIA one
+    clspmv::device_release(dia.dia_offsets, true);   // the DIA data array becomes the BDIA one
     dst->matinfo = dia.matinfo;
     dst->bdia_band_num = (int)first.size();
     dst->bdia_length = dia.dia_length;

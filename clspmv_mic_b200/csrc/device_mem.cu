@@ -1,4 +1,4 @@
-// device_mem.cu — upload / device_free entry points: cudaMalloc + copy of
+// device_mem.cu — upload / device_free entry points: a device array for, and a copy of,
 // every array of a host format struct into a device copy of the struct.
 // They replace the ALLOCATE_GPU_READ uploads of the reference drivers
 // (include/oclcommon.h:13-38) and cpy_<fmt>_mat of src/spmv_cocktail.cpp.
@@ -17,13 +17,10 @@ int upload_array(T** dst, const T* src, size_t n)
     if (n == 0) return CLSPMV_OK;
     if (!src) return CLSPMV_ERR_ARG;
     void* p = nullptr;
-    if (cudaMalloc(&p, n * sizeof(T)) != cudaSuccess) {
-        cudaGetLastError();
-        return CLSPMV_ERR_ALLOC;
-    }
+    if (clspmv::device_alloc(&p, n * sizeof(T))) return CLSPMV_ERR_ALLOC;
     int rc = cuda_status(cudaMemcpy(p, src, n * sizeof(T), cudaMemcpyHostToDevice));
     if (rc) {
-        cudaFree(p);
+        clspmv::device_release(p, false);
         return rc;
     }
     *dst = static_cast<T*>(p);
@@ -33,7 +30,7 @@ int upload_array(T** dst, const T* src, size_t n)
 template <class T>
 void release(T*& p)
 {
-    if (p) cudaFree(p);
+    clspmv::device_release(p, false);
     p = nullptr;
 }
 
@@ -53,7 +50,7 @@ struct Uploader {
     {
         if (rc)
             for (int i = 0; i < n; i++)
-                if (done[i]) cudaFree(done[i]);
+                clspmv::device_release(done[i], false);
         return rc;
     }
 };

@@ -410,7 +410,7 @@ def _computable(fmt: str) -> None:
 
 
 class _DeviceArrays:
-    """Arrays a device converter cudaMalloc'ed, released with
+    """Arrays a device converter made, released with
     clspmv_device_free_<fmt>_f32 when the last tensor viewing them is gone."""
 
     def __init__(self, fmt: str, struct):
@@ -503,6 +503,12 @@ def device_convert(coo: DeviceMatrix, fmt: str, *args, stream=None) -> DeviceMat
     self.stored_bytes = int(sum(t.numel() * t.element_size() for t in self.tensors.values()))
     self._owner = owner
     return self
+
+
+def device_trim() -> None:
+    """Gives back the released device arrays that the library keeps for its
+    next conversion or upload (clspmv_device_trim)."""
+    check(lib().clspmv_device_trim(), "device_trim")
 
 
 def device_sort_coo(coo: DeviceMatrix, stream=None) -> DeviceMatrix:

@@ -251,8 +251,12 @@ void clspmv_free_b4ell_f32(clspmv_b4ell_f32* m);
 void clspmv_free_sbell_f32(clspmv_sbell_f32* m);
 
 /* ------------------------------------------------------------------------ */
-/* Device residency. upload: cudaMalloc + copy of every array of `host`     */
-/* into `dev` (scalars copied). device_free: cudaFree of those arrays.      */
+/* Device residency. upload: a device array for, and a copy of, every array */
+/* of `host` into `dev` (scalars copied). device_free: waits for the device */
+/* and releases those arrays; a bounded number of released ones (1/64 of a  */
+/* device's memory) is kept for the next upload or conversion and given     */
+/* back by clspmv_device_trim, when an allocation of this library fails, or */
+/* when under 1/8 of the device is left after a large new one.              */
 /* Replaces the ALLOCATE_GPU_READ uploads of the per-format drivers         */
 /* (include/oclcommon.h:13-38) and the cpy_<fmt>_mat helpers of             */
 /* src/spmv_cocktail.cpp:304-1009.                                          */
@@ -279,10 +283,12 @@ int clspmv_device_free_bcsr_f32(clspmv_bcsr_f32* dev);
 int clspmv_device_free_bell_f32(clspmv_bell_f32* dev);
 int clspmv_device_free_b4ell_f32(clspmv_b4ell_f32* dev);
 int clspmv_device_free_sbell_f32(clspmv_sbell_f32* dev);
+/* Gives every kept released array of every device back (cudaFree). */
+int clspmv_device_trim(void);
 
 /* ------------------------------------------------------------------------ */
 /* Converters on the device. `coo` holds device arrays; the output struct   */
-/* gets cudaMalloc'ed device arrays (release with clspmv_device_free_<fmt>) */
+/* gets device arrays of its own (release with clspmv_device_free_<fmt>)    */
 /* equal byte for byte to what the host converter of the same name without  */
 /* `device_` makes from the same COO, with the same statuses (argument      */
 /* checks, CLSPMV_ERR_NOT_SORTED, refusals). The COO is not modified. Each  */

@@ -1,7 +1,12 @@
 """Device converters where their kernels change path: runs of empty rows of
 every listed length, block rows cut into several items, ranges too long to
 stage, arrays off a 16-byte boundary, alignments that leave strips off a
-4-value boundary. Each result equals the host converter's, byte for byte."""
+4-value boundary. Each result equals the host converter's, byte for byte.
+Released arrays are kept for the next call, given back by device_trim, and
+never handed out twice."""
+import ctypes as C
+import threading
+
 import numpy as np
 import pytest
 
@@ -81,3 +86,36 @@ def test_arrays_off_a_16_byte_boundary(fmt, args):
     got, (_, host) = F.device_convert(off, fmt, *args), host_raw(fmt, coo, *args)
     for field, _, _ in _abi.FORMATS[fmt][1]:
         assert np.array_equal(got.tensors[field].cpu().numpy().view(np.uint32), host.array(field).view(np.uint32)), field
+
+
+def test_released_arrays_are_handed_out_once():
+    """A struct freed through two copies of itself, and two threads converting
+    and dropping at once: every result stays the host's."""
+    coo = _case("mixed")
+    st, out = F.device_convert_raw(device_coo(coo), "csr")
+    assert st == _abi.OK
+    twice = _abi.Csr.from_buffer_copy(out)
+    F.lib().clspmv_device_free_csr_f32(C.byref(out))
+    F.lib().clspmv_device_free_csr_f32(C.byref(twice))
+    a, b = (F.device_convert(device_coo(coo), "csr") for _ in range(2))
+    ptrs = [t.data_ptr() for m in (a, b) for t in m.tensors.values()]
+    assert len(set(ptrs)) == len(ptrs)
+    _, host = host_raw("sell", coo)
+    wrong = []
+
+    def work():
+        s = torch.cuda.Stream()
+        with torch.cuda.stream(s):
+            dev = device_coo(coo)
+            for _ in range(20):
+                m = F.device_convert(dev, "sell")
+                if not np.array_equal(m.tensors["sell_data"].cpu().numpy(), host.array("sell_data")):
+                    wrong.append(1)
+                del m
+
+    threads = [threading.Thread(target=work) for _ in range(2)]
+    [t.start() for t in threads]
+    [t.join() for t in threads]
+    assert not wrong
+    F.device_trim()
+    check_pair("sell", coo)
