@@ -10,9 +10,8 @@
 // aligned, else 1), so every stored element of A is read once per group and
 // multiplies one contiguous row of X. The regular formats (DIA, BDIA, ELL,
 // SELL, b4csr, b4ell, SBELL) walk their own layout row by row; CSR and COO
-// split the nonzeros into equal chunks per group (power-law rows cost the
-// same as short ones) and add the partial sums of rows cut by a chunk edge
-// with vector atomics.
+// split the nonzeros into equal runs per warp (power-law rows cost the same
+// as short ones; k_spmm_runs).
 //
 // Reduced-precision storage: clspmv_pack_values converts a device matrix's
 // FP32 values in place of a caller-supplied 16-bit array: every value of row
@@ -177,6 +176,10 @@ template <> struct Acc<1> {
         *y = beta == 0.0f ? alpha * v : fmaf(beta, *y, alpha * v);
     }
     __device__ void add(float* y, float alpha) const { *y += alpha * v; }
+    __device__ void store_cs(float* y, float alpha, float beta) const
+    {
+        __stcs(y, beta == 0.0f ? alpha * v : fmaf(beta, *y, alpha * v));
+    }
     __device__ void atomic(float* y, float alpha) const { atomicAdd(y, alpha * v); }
 };
 template <> struct Acc<4> {
@@ -220,6 +223,7 @@ template <> struct Acc<4> {
         p.w += alpha * v.w;
         *reinterpret_cast<float4*>(y) = p;
     }
+    __device__ void store_cs(float* y, float alpha, float beta) const { store(y, alpha, beta); }
     __device__ void atomic(float* y, float alpha) const
     {
         atomicAdd(reinterpret_cast<float4*>(y), make_float4(alpha * v.x, alpha * v.y, alpha * v.z, alpha * v.w));
@@ -396,111 +400,8 @@ __global__ void __launch_bounds__(kSpmmBlock, BH >= 8 ? 1 : 4) k_spmm_blocks(M m
         block_row<BH, BW4>(m, vals, (int)br, c0, d.X, d.ldx, d.Y, d.ldy, d.alpha, d.beta, d.scale, d.x_form);
 }
 
-// Nonzero-chunk kernel for CSR (row_ptr) and row-sorted COO (row_id). Y must
-// already hold beta * Y. A row wholly inside a chunk is added with a plain
-// read-modify-write; a row cut by a chunk edge is added atomically.
-constexpr int kChunkPrefetch = 4;
-
-template <int VEC, class T, bool IS_CSR>
-__global__ void __launch_bounds__(kSpmmBlock) k_spmm_chunks(int rows, int nnz, const int* __restrict__ row_ptr,
-                                                            const int* __restrict__ row_id, const int* __restrict__ col_id,
-                                                            const T* __restrict__ vals, int chunk, Dense d)
-{
-    const int G = 1 << d.lshift;
-    const long long t = (long long)blockIdx.x * kSpmmBlock + threadIdx.x;
-    const int lane = (int)(t & (G - 1));
-    const int c0 = lane * VEC;
-    if (c0 >= d.k) return;
-    const long long g = t >> d.lshift;
-    const long long e0l = g * chunk;
-    if (e0l >= nnz) return;
-    const int e0 = (int)e0l;
-    const int e1 = (int)min((long long)nnz, e0l + chunk);
-    int row, row_end = 0;
-    if (IS_CSR) {   // last row whose start is <= e0 (skips empty rows)
-        int lo = 0, hi = rows;
-        while (lo < hi) {
-            const int mid = (lo + hi + 1) >> 1;
-            if (__ldg(row_ptr + mid) <= e0) lo = mid;
-            else hi = mid - 1;
-        }
-        row = lo;
-        row_end = __ldg(row_ptr + row + 1);
-    } else {
-        row = __ldg(row_id + e0);
-    }
-    bool first = true;   // the current row may have started before e0
-    Acc<VEC> acc;
-    // A row is cut by the chunk if it started before e0 (only the first row
-    // can) or continues past e1 (only the last row can).
-    auto flush = [&](bool last) {
-        const float a = d.scale ? d.alpha * d.scale[row] : d.alpha;
-        float* y = d.Y + (size_t)row * d.ldy + c0;
-        bool cut = false;
-        if (first) cut = IS_CSR ? __ldg(row_ptr + row) < e0 : (e0 > 0 && __ldg(row_id + e0 - 1) == row);
-        if (last) cut = cut || (IS_CSR ? row_end > e1 : (e1 < nnz && __ldg(row_id + e1) == row));
-        if (cut) acc.atomic(y, a);
-        else acc.add(y, a);
-    };
-    // kChunkPrefetch nonzeros at a time: their column ids, values and X
-    // slices are all requested before the first is used, so a lane keeps
-    // that many gathers in flight
-    constexpr int U = kChunkPrefetch;
-    for (int e = e0; e < e1; e += U) {
-        int cc[U], rr[U];
-        float vv[U];
-        typename Acc<VEC>::X xv[U];
-#pragma unroll
-        for (int u = 0; u < U; u++) {
-            const bool in = e + u < e1;
-            cc[u] = in ? __ldg(col_id + e + u) : 0;
-            vv[u] = in ? to_f(ld_val(vals + e + u)) : 0.f;
-            rr[u] = (!IS_CSR && in) ? __ldg(row_id + e + u) : 0;
-        }
-#pragma unroll
-        for (int u = 0; u < U; u++) xv[u] = e + u < e1 ? Acc<VEC>::load(d.X + (size_t)cc[u] * d.ldx + c0) : Acc<VEC>::zero();
-#pragma unroll
-        for (int u = 0; u < U; u++) {
-            const int ee = e + u;
-            if (ee >= e1) break;
-            if (IS_CSR) {
-                if (ee >= row_end) {
-                    flush(false);
-                    first = false;
-                    acc = Acc<VEC>();
-                    do {
-                        row++;
-                        row_end = __ldg(row_ptr + row + 1);
-                    } while (ee >= row_end);
-                }
-            } else if (rr[u] != row) {
-                flush(false);
-                first = false;
-                acc = Acc<VEC>();
-                row = rr[u];
-            }
-            acc.fma_v(vv[u], xv[u]);
-        }
-    }
-    flush(true);
-}
-
-// ---------------------------------------------------------------------------
-// Warp-segmented CSR / COO product for k a multiple of 4 (used at k = 4)
-// with 16-byte rows of X and Y: the mapping of the single-vector COO kernel (a warp per 256
-// consecutive nonzeros, 4 per lane, all of a step's X gathers issued at
-// once) applied to each group of 4 columns in turn, with float4 partial sums
-// reduced by the same per-lane runs + warp segmented scan and added to Y with
-// vector red.global.add. The nonzero-chunk kernel above walks a chunk's
-// nonzeros one after another per lane group; this one keeps 8 gathers of 16
-// bytes in flight per lane. CSR rows come from row_ptr: a warp-wide 32-way
-// search finds the first and last row of the chunk, each lane then searches
-// between them. Y must already hold beta * Y.
-// ---------------------------------------------------------------------------
 constexpr unsigned kWarpAll = 0xffffffffu;
 constexpr int kSegNoRow = 0x7fffffff;
-constexpr int kSegSteps = 2;
-constexpr int kSegChunk = 128 * kSegSteps;
 
 __device__ __forceinline__ float4 f4add(float4 a, float4 b) { return make_float4(a.x + b.x, a.y + b.y, a.z + b.z, a.w + b.w); }
 __device__ __forceinline__ float4 f4up(float4 v, int off)
@@ -508,12 +409,6 @@ __device__ __forceinline__ float4 f4up(float4 v, int off)
     return make_float4(__shfl_up_sync(kWarpAll, v.x, off), __shfl_up_sync(kWarpAll, v.y, off),
                        __shfl_up_sync(kWarpAll, v.z, off), __shfl_up_sync(kWarpAll, v.w, off));
 }
-__device__ __forceinline__ float4 f4from(float4 v, int src)
-{
-    return make_float4(__shfl_sync(kWarpAll, v.x, src), __shfl_sync(kWarpAll, v.y, src), __shfl_sync(kWarpAll, v.z, src),
-                       __shfl_sync(kWarpAll, v.w, src));
-}
-
 // Largest r in [0, rows) with row_ptr[r] <= q (q < nnz), by the whole warp:
 // each round the 32 lanes probe 32 evenly spaced rows of the interval.
 __device__ __forceinline__ int warp_row_of(const int* __restrict__ row_ptr, int rows, long long q, int lane)
@@ -534,177 +429,6 @@ __device__ __forceinline__ int warp_row_of(const int* __restrict__ row_ptr, int 
     return lo + (31 - __clz(m));
 }
 
-__device__ __forceinline__ void seg_red(const Dense& d, int row, int c0, float4 v)
-{
-    if (row == kSegNoRow) return;
-    const float a = d.scale ? d.alpha * d.scale[row] : d.alpha;
-    atomicAdd(reinterpret_cast<float4*>(d.Y + (size_t)row * d.ldy + c0), make_float4(a * v.x, a * v.y, a * v.z, a * v.w));
-}
-
-// The segmented reduction of the COO kernel (per-lane runs, lane-boundary
-// partials by a warp scan, the trailing row carried across steps) on float4
-// sums of 4 columns.
-__device__ __forceinline__ void seg_reduce4(const Dense& d, int c0, const int (&r)[kSegSteps][4],
-                                            const float4 (&p)[kSegSteps][4], int lane)
-{
-    const float4 zero = make_float4(0.f, 0.f, 0.f, 0.f);
-    float4 carry = zero;
-    int carry_row = -1;
-#pragma unroll
-    for (int s = 0; s < kSegSteps; s++) {
-        const int head_row = r[s][0], tail_row = r[s][3];
-        const bool single = head_row == tail_row;
-        float4 head = zero, tail = zero;
-        if (single) {
-            tail = f4add(f4add(p[s][0], p[s][1]), f4add(p[s][2], p[s][3]));
-        } else {
-            head = p[s][0];
-            tail = p[s][3];
-            int run_row = -1;
-            float4 run = zero;
-#pragma unroll
-            for (int j = 1; j < 3; j++) {
-                const int rj = r[s][j];
-                if (rj == head_row) {
-                    head = f4add(head, p[s][j]);
-                } else if (rj == tail_row) {
-                    tail = f4add(tail, p[s][j]);
-                } else if (rj == run_row) {
-                    run = f4add(run, p[s][j]);
-                } else {
-                    if (run_row >= 0) seg_red(d, run_row, c0, run);
-                    run_row = rj;
-                    run = p[s][j];
-                }
-            }
-            if (run_row >= 0) seg_red(d, run_row, c0, run);
-        }
-        const int lead = __shfl_sync(kWarpAll, head_row, 0);
-        if (carry_row >= 0 && lead != carry_row) {
-            if (lane == 0) seg_red(d, carry_row, c0, carry);
-            carry_row = -1;
-            carry = zero;
-        }
-        if (lane == 0 && carry_row >= 0) {
-            if (single) tail = f4add(tail, carry);
-            else head = f4add(head, carry);
-        }
-        const int prev_tail_row = __shfl_up_sync(kWarpAll, tail_row, 1);
-        const bool start = lane == 0 || !single || prev_tail_row != tail_row;
-        const unsigned smask = __ballot_sync(kWarpAll, start);
-        const int seg0 = 31 - __clz(smask & (0xffffffffu >> (31 - lane)));
-        float4 v = tail;
-#pragma unroll
-        for (int off = 1; off < 32; off <<= 1) {
-            const float4 t = f4up(v, off);
-            if (lane - off >= seg0) v = f4add(v, t);
-        }
-        const float4 prev_v = f4up(v, 1);
-        if (!single) seg_red(d, head_row, c0, (lane > 0 && prev_tail_row == head_row) ? f4add(head, prev_v) : head);
-        const int next_head = __shfl_down_sync(kWarpAll, head_row, 1);
-        if (lane < 31 && next_head != tail_row) seg_red(d, tail_row, c0, v);
-        carry = f4from(v, 31);
-        carry_row = __shfl_sync(kWarpAll, tail_row, 31);
-        if (carry_row == kSegNoRow) carry_row = -1;
-    }
-    if (carry_row >= 0 && lane == 0) seg_red(d, carry_row, c0, carry);
-}
-
-template <class T, bool IS_CSR>
-__device__ __forceinline__ void seg_chunk(int rows, int nnz, const int* __restrict__ row_ptr, const int* __restrict__ row_id,
-                                          const int* __restrict__ col_id, const T* __restrict__ vals, const Dense& d,
-                                          long long ch, int lane)
-{
-    const long long base = ch * kSegChunk;
-    int r[kSegSteps][4], c[kSegSteps][4];
-    float v[kSegSteps][4];
-#pragma unroll
-    for (int s = 0; s < kSegSteps; s++) {
-        const long long idx = base + s * 128 + lane * 4;
-        if (idx + 3 < nnz) {
-            const int4 cv = __ldg(reinterpret_cast<const int4*>(col_id + idx));
-            c[s][0] = cv.x; c[s][1] = cv.y; c[s][2] = cv.z; c[s][3] = cv.w;
-            if constexpr (std::is_same<T, float>::value) {
-                const float4 vv = __ldg(reinterpret_cast<const float4*>(vals + idx));
-                v[s][0] = vv.x; v[s][1] = vv.y; v[s][2] = vv.z; v[s][3] = vv.w;
-            } else {
-#pragma unroll
-                for (int j = 0; j < 4; j++) v[s][j] = to_f(ld_val(vals + idx + j));
-            }
-            if (!IS_CSR) {
-                const int4 rv = __ldg(reinterpret_cast<const int4*>(row_id + idx));
-                r[s][0] = rv.x; r[s][1] = rv.y; r[s][2] = rv.z; r[s][3] = rv.w;
-            }
-        } else {
-#pragma unroll
-            for (int j = 0; j < 4; j++) {
-                const bool in = idx + j < nnz;
-                c[s][j] = in ? __ldg(col_id + idx + j) : 0;
-                v[s][j] = in ? to_f(ld_val(vals + idx + j)) : 0.f;
-                if (!IS_CSR) r[s][j] = in ? __ldg(row_id + idx + j) : kSegNoRow;
-            }
-        }
-    }
-    if (IS_CSR) {
-        const int ra = warp_row_of(row_ptr, rows, base, lane);
-        const int rb = warp_row_of(row_ptr, rows, min(base + kSegChunk - 1, (long long)nnz - 1), lane);
-#pragma unroll
-        for (int s = 0; s < kSegSteps; s++) {
-            const long long q0 = base + s * 128 + lane * 4;
-            if (q0 >= nnz) {
-#pragma unroll
-                for (int j = 0; j < 4; j++) r[s][j] = kSegNoRow;
-                continue;
-            }
-            int lo = ra, hi = rb;
-            while (lo < hi) {
-                const int mid = (lo + hi + 1) >> 1;
-                if (__ldg(row_ptr + mid) <= q0) lo = mid;
-                else hi = mid - 1;
-            }
-            int row = lo;
-            r[s][0] = row;
-#pragma unroll
-            for (int j = 1; j < 4; j++) {
-                const long long q = q0 + j;
-                if (q < nnz) {
-                    while (__ldg(row_ptr + row + 1) <= q) row++;
-                    r[s][j] = row;
-                } else {
-                    r[s][j] = kSegNoRow;
-                }
-            }
-        }
-    }
-    for (int c0 = 0; c0 < d.k; c0 += 4) {
-        float4 p[kSegSteps][4];
-#pragma unroll
-        for (int s = 0; s < kSegSteps; s++)
-#pragma unroll
-            for (int j = 0; j < 4; j++) {
-                if (r[s][j] != kSegNoRow) {
-                    const float4 xv = __ldg(reinterpret_cast<const float4*>(d.X + (size_t)c[s][j] * d.ldx + c0));
-                    p[s][j] = make_float4(v[s][j] * xv.x, v[s][j] * xv.y, v[s][j] * xv.z, v[s][j] * xv.w);
-                } else {
-                    p[s][j] = make_float4(0.f, 0.f, 0.f, 0.f);
-                }
-            }
-        seg_reduce4(d, c0, r, p, lane);
-    }
-}
-
-template <class T, bool IS_CSR>
-__global__ void __launch_bounds__(kSpmmBlock) k_spmm_seg(int rows, int nnz, const int* __restrict__ row_ptr,
-                                                         const int* __restrict__ row_id, const int* __restrict__ col_id,
-                                                         const T* __restrict__ vals, Dense d)
-{
-    const int lane = threadIdx.x & 31;
-    const long long nchunks = ((long long)nnz + kSegChunk - 1) / kSegChunk;
-    const long long nwarps = (long long)gridDim.x * (kSpmmBlock / 32);
-    for (long long ch = (long long)blockIdx.x * (kSpmmBlock / 32) + (threadIdx.x >> 5); ch < nchunks; ch += nwarps)
-        seg_chunk<T, IS_CSR>(rows, nnz, row_ptr, row_id, col_id, vals, d, ch, lane);
-}
-
 // ---------------------------------------------------------------------------
 // Long CSR rows at k a multiple of 4: a warp per row. The warp's lanes form
 // 32 / G nonzero slots of G = k / 4 lanes (4 columns each); a step covers
@@ -712,8 +436,7 @@ __global__ void __launch_bounds__(kSpmmBlock) k_spmm_seg(int rows, int nnz, cons
 // and one float4 X load per lane, and the slots' partial sums are combined
 // once per row by shuffles. The row is owned by its warp, so Y is written
 // directly (alpha, beta applied there). Used when rows average
-// kWarpRowMin nonzeros or more: the nonzero-chunk kernel walks a long row's
-// nonzeros one after another per lane group.
+// kWarpRowMin nonzeros or more.
 // ---------------------------------------------------------------------------
 constexpr int kWarpRowMin = 128;
 
@@ -767,6 +490,271 @@ __global__ void __launch_bounds__(kSpmmBlock) k_spmm_warp_rows(int rows, const i
             }
             *y = o;
         }
+    }
+}
+
+// ---------------------------------------------------------------------------
+// CSR / COO by warp runs. A warp takes 32 P consecutive nonzeros, P per lane
+// with 128-bit loads, finds the row of each (CSR: from row_ptr), and splits
+// its lanes into slots of G = 2^LG lanes that share the k columns of X and Y
+// (VEC columns a lane). A slot owns the P G nonzeros that its lanes loaded
+// and hands them round by shuffles, with kRunLoads X rows in flight: ids,
+// values and rows are read once, coalesced, and no lane waits for row_ptr
+// between two nonzeros.
+//
+// A CSR row that starts and ends in its warp's run is written directly
+// (alpha, beta), its pieces in several slots summed by a segmented scan, so
+// Y gets no scaling pass of its own. Only rows cut by an edge between warps
+// are added atomically, after k_scale_cut has applied beta to those and to
+// the rows without entries. COO has no row pointer to tell them by: beta is
+// applied to all of Y first and every row is added, by red.global.add, which
+// a slot does not wait for.
+//
+// Measured on B200 (us, CSR, FP32; before: 16 nonzeros per lane group, a
+// search of row_ptr for each, Y zeroed first and every row read, added and
+// written): power law of 2^20 rows, k = 4 / 16 / 32: 186 / 325 / 566 -> 105 /
+// 197 / 345; 27-point stencil of 100^3: 266 / 376 / 621 -> 127 / 250 / 432.
+// At k = 16 on the power law it moves its 1.04 GB of X rows at 5.3 TB/s (X is
+// 64 MB: L2 hits 57 %), at k = 64 at 6.4 TB/s, the rate of DRAM. Also measured, not
+// kept: rows walked within equal ranges of nonzeros, several slots a row
+// (358 us at k = 16 on the power law), ends of rows written without a branch
+// (280), evict-last X or streaming Y (within 3 %), 3 CTAs per SM (198).
+// ---------------------------------------------------------------------------
+constexpr int kRunLoads = 4;
+
+// beta to the rows that an edge between warp runs of `run` nonzeros cuts, and to rows without entries.
+__global__ void __launch_bounds__(kSpmmBlock) k_scale_cut(int rows, const int* __restrict__ row_ptr, int run, Dense d)
+{
+    for (long long r = (long long)blockIdx.x * kSpmmBlock + threadIdx.x; r < rows; r += (long long)gridDim.x * kSpmmBlock) {
+        const int s = __ldg(row_ptr + r), e = __ldg(row_ptr + r + 1);
+        if (s < e && s / run == (e - 1) / run) continue;
+        float* y = d.Y + (size_t)r * d.ldy;
+        for (int j = 0; j < d.k; j++) y[j] = d.beta == 0.0f ? 0.0f : d.beta * y[j];
+    }
+}
+
+// The row that holds nonzero e, the current row having ended at or before it.
+__device__ __forceinline__ int next_row(const int* __restrict__ row_ptr, int rows, int row, int e)
+{
+    for (int i = 0; i < 8; i++) {
+        row++;
+        if (__ldg(row_ptr + row + 1) > e) return row;
+    }
+    int lo = row + 1, hi = rows - 1;   // many rows without entries: the largest row that starts at or before e
+    while (lo < hi) {
+        const int mid = lo + ((hi - lo + 1) >> 1);
+        if (__ldg(row_ptr + mid) <= e) lo = mid;
+        else hi = mid - 1;
+    }
+    return lo;
+}
+
+// Rows of a lane's P nonzeros from q0 on (kSegNoRow past the last one), q0 in [base, ...), ra the
+// row of base. The rows of most runs lie within 256 of ra: every eighth of
+// those row pointers is held by one lane, so a lane searches by shuffles and
+// then among 8. Otherwise it searches up to the last row.
+template <int P>
+__device__ __forceinline__ void rows_of(const int* __restrict__ row_ptr, int rows, int ra, long long q0, int end, int lane, int (&r)[P])
+{
+    const int probe = min((long long)ra + 8 * lane, (long long)rows);   // row_ptr[rows] = nnz is past every q
+    const int pv = __ldg(row_ptr + probe);
+    const bool near = __shfl_sync(kWarpAll, pv, 31) >= end;   // the rows of the run end before the last probe
+    const long long q = min(q0, (long long)end - 1);
+    int lo, hi;
+    if (near) {
+        int j = 0;
+#pragma unroll
+        for (int s = 16; s > 0; s >>= 1) {
+            const int v = __shfl_sync(kWarpAll, pv, j + s);
+            if (v <= q) j += s;
+        }
+        lo = ra + 8 * j;
+        hi = min(lo + 7, rows - 1);
+    } else {
+        lo = ra;
+        hi = rows - 1;
+    }
+    while (lo < hi) {
+        const int mid = lo + ((hi - lo + 1) >> 1);
+        if (__ldg(row_ptr + mid) <= q) lo = mid;
+        else hi = mid - 1;
+    }
+    int row = lo, next = __ldg(row_ptr + row + 1);
+#pragma unroll
+    for (int j = 0; j < P; j++) {
+        const long long e = q0 + j;
+        if (e < end) {
+            if (e >= next) {
+                row = next_row(row_ptr, rows, row, (int)e);
+                next = __ldg(row_ptr + row + 1);
+            }
+            r[j] = row;
+        } else {
+            r[j] = kSegNoRow;
+        }
+    }
+}
+
+template <class T, int P>
+__device__ __forceinline__ void load_run(const T* __restrict__ p, long long i, int nnz, bool vec, float (&v)[P])
+{
+    if (vec && i + P <= nnz) {
+        if constexpr (std::is_same<T, float>::value) {
+#pragma unroll
+            for (int j = 0; j < P; j += 4) {
+                const float4 f = __ldcs(reinterpret_cast<const float4*>(p + i + j));
+                v[j] = f.x; v[j + 1] = f.y; v[j + 2] = f.z; v[j + 3] = f.w;
+            }
+        } else {
+#pragma unroll
+            for (int j = 0; j < P; j += 4) {
+                const uint2 u = __ldcs(reinterpret_cast<const uint2*>(p + i + j));
+                const T* t = reinterpret_cast<const T*>(&u);
+#pragma unroll
+                for (int q = 0; q < 4; q++) v[j + q] = to_f(t[q]);
+            }
+        }
+    } else {
+#pragma unroll
+        for (int j = 0; j < P; j++) v[j] = i + j < nnz ? to_f(ld_val(p + i + j)) : 0.f;
+    }
+}
+template <int P>
+__device__ __forceinline__ void load_ids(const int* __restrict__ p, long long i, int nnz, bool vec, int (&c)[P])
+{
+    if (vec && i + P <= nnz) {
+#pragma unroll
+        for (int j = 0; j < P; j += 4) {
+            const int4 f = __ldcs(reinterpret_cast<const int4*>(p + i + j));
+            c[j] = f.x; c[j + 1] = f.y; c[j + 2] = f.z; c[j + 3] = f.w;
+        }
+    } else {
+#pragma unroll
+        for (int j = 0; j < P; j++) c[j] = i + j < nnz ? __ldg(p + i + j) : 0;
+    }
+}
+
+__device__ __forceinline__ float shfl_up_x(float v, int o) { return __shfl_up_sync(kWarpAll, v, o); }
+__device__ __forceinline__ float4 shfl_up_x(float4 v, int o) { return f4up(v, o); }
+__device__ __forceinline__ float x_add(float a, float b) { return a + b; }
+__device__ __forceinline__ float4 x_add(float4 a, float4 b) { return f4add(a, b); }
+
+template <int LG, int VEC, int P, class T, bool IS_CSR>
+__global__ void __launch_bounds__(kSpmmBlock, 4) k_spmm_runs(int rows, int nnz, const int* __restrict__ row_ptr,
+                                                             const int* __restrict__ row_id, const int* __restrict__ col_id,
+                                                             const T* __restrict__ vals, bool vec, int per, Dense d)
+{
+    constexpr int G = 1 << LG, kRun = 32 * P, U = kRunLoads;
+    static_assert(P % U == 0, "a batch of X rows stays within a lane's nonzeros");
+    using XT = typename Acc<VEC>::X;
+    const int lane = threadIdx.x & 31, slot = lane >> LG;
+    const int c0 = (lane & (G - 1)) * VEC;
+    const bool cols = c0 < d.k;
+    const float* __restrict__ X = d.X + (cols ? c0 : 0);
+    float* const Y = d.Y + c0;
+    // `per` consecutive runs per warp: the row of the next run's start is found from this one's
+    const long long w0 = ((long long)blockIdx.x * (kSpmmBlock / 32) + (threadIdx.x >> 5)) * per;
+    int ra = 0;
+    if (IS_CSR && w0 * kRun < nnz) ra = warp_row_of(row_ptr, rows, w0 * kRun, lane);
+    for (long long w = w0; w < w0 + per && w * kRun < nnz; w++) {
+        const int base = (int)(w * kRun), end = (int)min((long long)nnz, (w + 1) * kRun);
+        const long long q0 = base + (long long)lane * P;
+        int cc[P], rr[P];
+        float vv[P];
+        load_ids<P>(col_id, q0, nnz, vec, cc);
+        load_run<T, P>(vals, q0, nnz, vec, vv);
+        if (IS_CSR) {
+            rows_of<P>(row_ptr, rows, ra, q0, end, lane, rr);
+        } else {
+            load_ids<P>(row_id, q0, nnz, vec, rr);
+#pragma unroll
+            for (int j = 0; j < P; j++)
+                if (q0 + j >= nnz) rr[j] = kSegNoRow;
+        }
+        // the rows of the nonzeros before and after the slot's
+        int before = __shfl_up_sync(kWarpAll, rr[P - 1], 1), after = __shfl_down_sync(kWarpAll, rr[0], 1);
+        if (IS_CSR) {
+            if (lane == 0) before = __ldg(row_ptr + ra) < base ? ra : -1;
+            if (lane == 31) after = rr[P - 1] != kSegNoRow && __ldg(row_ptr + rr[P - 1] + 1) > end ? rr[P - 1] : kSegNoRow;
+        } else {
+            if (lane == 0) before = base > 0 ? __ldg(row_id + base - 1) : -1;
+            if (lane == 31) after = end < nnz ? __ldg(row_id + end) : kSegNoRow;
+        }
+        const int base_row = __shfl_sync(kWarpAll, before, 0);   // the row that came from before the warp, if any
+        before = __shfl_sync(kWarpAll, before, 0, G);
+        after = __shfl_sync(kWarpAll, after, G - 1, G);
+        int row = __shfl_sync(kWarpAll, rr[0], 0, G);
+        bool cut = row == before;    // the current row's sum is a piece
+        int head_row = -1;
+        Acc<VEC> acc, first;         // first: the piece of the row that the slot starts in, once that row has ended
+        auto put = [&](const Acc<VEC>& s, int r, bool whole) {
+            float a = d.alpha;
+            if (!std::is_same<T, float>::value) a *= d.scale[r];
+            float* y = Y + (size_t)r * d.ldy;
+            if (!IS_CSR || !whole) s.atomic(y, a);
+            else if (VEC == 1) s.store_cs(y, a, d.beta);
+            else s.store(y, a, d.beta);
+        };
+        auto row_done = [&]() {
+            if (cut) {
+                first = acc;
+                head_row = row;
+                cut = false;
+            } else if (cols) {
+                put(acc, row, true);
+            }
+            acc = Acc<VEC>();
+        };
+#pragma unroll 1
+        for (int src = 0; src < G; src++) {
+#pragma unroll
+            for (int h = 0; h < P; h += U) {
+                float av[U];
+                int rv[U];
+                XT xv[U];
+#pragma unroll
+                for (int u = 0; u < U; u++) {
+                    const int c = __shfl_sync(kWarpAll, cc[h + u], src, G);
+                    av[u] = __shfl_sync(kWarpAll, vv[h + u], src, G);
+                    rv[u] = __shfl_sync(kWarpAll, rr[h + u], src, G);
+                    xv[u] = cols && rv[u] != kSegNoRow ? Acc<VEC>::load(X + (size_t)c * d.ldx) : Acc<VEC>::zero();
+                }
+#pragma unroll
+                for (int u = 0; u < U; u++) {
+                    if (rv[u] != row) {
+                        row_done();
+                        row = rv[u];
+                        if (row == kSegNoRow) cut = true;   // past the last nonzero: nothing is written from here on
+                    }
+                    acc.fma_v(av[u], xv[u]);
+                }
+            }
+        }
+        // the slot's last row: done here, or continued in the next slot
+        const bool live = row != kSegNoRow, more = live && row == after;
+        if (live && !more) row_done();
+        // pieces, in slot order: a slot inside one row hands the sum on (through), others start a new one with their last row's piece
+        const bool through = more && cut;
+        XT v = more ? acc.v : Acc<VEC>::zero();
+        const unsigned upto = __ballot_sync(kWarpAll, !through) & (0xffffffffu >> (31 - lane));
+        const int seg0 = upto ? (31 - __clz(upto)) & ~(G - 1) : 0;   // first lane of the slot where this slot's sum starts
+#pragma unroll
+        for (int o = G; o < 32; o <<= 1) {
+            const XT t = shfl_up_x(v, o);
+            if (lane - o >= seg0) v = x_add(v, t);
+        }
+        XT pv = v;
+        if (G < 32) pv = shfl_up_x(v, G);
+        if (head_row >= 0 && head_row != kSegNoRow && cols) {   // a row that came from before ends in this slot
+            if (slot > 0) first.v = x_add(first.v, pv);
+            put(first, head_row, head_row != base_row);
+        }
+        if (more && lane >= 32 - G && cols) {                   // a row that goes on in the next warp's run
+            acc.v = v;
+            put(acc, row, false);
+        }
+        if (IS_CSR) ra = __shfl_sync(kWarpAll, after != kSegNoRow ? after : row, 31);
+        if (IS_CSR && end < nnz && __shfl_sync(kWarpAll, after, 31) == kSegNoRow) ra = next_row(row_ptr, rows, ra, end);
     }
 }
 
@@ -961,44 +949,50 @@ bool warp_rows_enabled()
     return on;
 }
 
-// CLSPMV_SPMM_SEG=0 keeps the nonzero-chunk kernel for CSR / COO (measurements).
-bool seg_enabled()
+template <int LG, int VEC, int P, class T, bool IS_CSR>
+void launch_runs(int rows, int nnz, const int* row_ptr, const int* row_id, const int* col_id, const T* v, bool vec, Dense d,
+                 cudaStream_t st)
 {
-    static const bool on = [] {
-        const char* e = getenv("CLSPMV_SPMM_SEG");
-        return !(e && atoi(e) == 0);
-    }();
-    return on;
+    const long long runs = ((long long)nnz + 32 * P - 1) / (32 * P), wpb = kSpmmBlock / 32;
+    const long long resident = 148LL * 4 * wpb;
+    const long long per = (runs + resident - 1) / resident;   // 1 while the runs do not fill the device
+    const int grid = (int)((runs + per * wpb - 1) / (per * wpb));
+    k_spmm_runs<LG, VEC, P, T, IS_CSR><<<grid, kSpmmBlock, 0, st>>>(rows, nnz, row_ptr, row_id, col_id, v, vec, (int)per, d);
 }
 
 template <class T, bool IS_CSR>
 int launch_chunks(int rows, int nnz, const int* row_ptr, const int* row_id, const int* col_id, const void* vals, Dense d,
                   int vec, cudaStream_t st)
 {
+    // 8 nonzeros per lane from where their runs fill the device's warps (1.2M nonzeros): 4 loses up to 1.4x there
+    // at k <= 16 (more searches and scans a nonzero) and wins 1.1-1.4x on 0.24M nonzeros (more warps)
+    const bool few = nnz < 148 * 32 * 256;
     if (d.beta != 1.0f) {
-        k_scale_rows<<<grid_of((long long)rows * d.k), kSpmmBlock, 0, st>>>(d.Y, rows, d.k, d.ldy, d.beta);
+        if (IS_CSR && nnz > 0)
+            k_scale_cut<<<grid_of(rows), kSpmmBlock, 0, st>>>(rows, row_ptr, few ? 128 : 256, d);
+        else
+            k_scale_rows<<<grid_of((long long)rows * d.k), kSpmmBlock, 0, st>>>(d.Y, rows, d.k, d.ldy, d.beta);
         int rc = after_launch(1);
         if (rc) return rc;
     }
     if (nnz <= 0) return CLSPMV_OK;
-    // k = 4: the warp-segmented kernel (measured on the power-law matrix: CSR 0.19 against 0.26 ms, COO 0.12
-    // against 0.68 ms); from k = 8 on the per-column scans cost more than the lane-per-column walk saves
-    if (vec == 4 && d.k == 4 && seg_enabled() && ((uintptr_t)col_id & 15) == 0 && (IS_CSR || ((uintptr_t)row_id & 15) == 0) &&
-        (!std::is_same<T, float>::value || ((uintptr_t)vals & 15) == 0)) {
-        const long long nchunks = ((long long)nnz + kSegChunk - 1) / kSegChunk;
-        const int grid = (int)std::min<long long>((nchunks + kSpmmBlock / 32 - 1) / (kSpmmBlock / 32), 148LL * 8);
-        k_spmm_seg<T, IS_CSR><<<grid, kSpmmBlock, 0, st>>>(rows, nnz, row_ptr, row_id, col_id,
-                                                          static_cast<const T*>(vals), d);
-        return after_launch(1);
-    }
-    // about 16 row-sum updates of X per lane: enough work to hide the search
-    const int chunk = d.k <= 4 ? 32 : 16;
-    const long long groups = ((long long)nnz + chunk - 1) / chunk;
-    const long long threads = groups << d.lshift;
-    const int grid = (int)((threads + kSpmmBlock - 1) / kSpmmBlock);
     const T* v = static_cast<const T*>(vals);
-    if (vec == 4) k_spmm_chunks<4, T, IS_CSR><<<grid, kSpmmBlock, 0, st>>>(rows, nnz, row_ptr, row_id, col_id, v, chunk, d);
-    else k_spmm_chunks<1, T, IS_CSR><<<grid, kSpmmBlock, 0, st>>>(rows, nnz, row_ptr, row_id, col_id, v, chunk, d);
+    const bool al = ((uintptr_t)col_id & 15) == 0 && (IS_CSR || ((uintptr_t)row_id & 15) == 0) && ((uintptr_t)v & (4 * sizeof(T) - 1)) == 0;
+#define RUNS(LG, VEC)                                                                                            \
+    case LG:                                                                                                     \
+        if (few) launch_runs<LG, VEC, 4, T, IS_CSR>(rows, nnz, row_ptr, row_id, col_id, v, al, d, st);           \
+        else launch_runs<LG, VEC, 8, T, IS_CSR>(rows, nnz, row_ptr, row_id, col_id, v, al, d, st);               \
+        break;
+    if (vec == 4) {
+        switch (d.lshift) {
+            RUNS(0, 4) RUNS(1, 4) RUNS(2, 4) RUNS(3, 4) RUNS(4, 4) RUNS(5, 4)
+        }
+    } else {
+        switch (d.lshift) {
+            RUNS(0, 1) RUNS(1, 1) RUNS(2, 1) RUNS(3, 1) RUNS(4, 1) RUNS(5, 1)
+        }
+    }
+#undef RUNS
     return after_launch(1);
 }
 
@@ -1195,7 +1189,7 @@ __device__ __forceinline__ void batch_blocks(const BatchJob& J, int br, int c0)
 
 // CSR job accumulating into Y: the group owns nonzeros [e0, e0 + chunk); rows
 // cut by the chunk's edges are added atomically, the others with a plain add
-// (as k_spmm_chunks, with Y already holding beta * Y = Y).
+// (Y already holds beta * Y = Y).
 template <int VEC, class T>
 __device__ __forceinline__ void batch_chunk(const BatchJob& J, int e0, int c0)
 {
