@@ -260,6 +260,74 @@ __global__ void __launch_bounds__(kSpmmBlock) k_spmm_rows(M m, const T* __restri
     }
 }
 
+// Row r of ELL and SELL: where its slot 0 lies, the step to the next, their number.
+__device__ __forceinline__ void slot_row(const clspmv_ell_f32& m, long long r, size_t& at, int& step, int& n)
+{
+    at = (size_t)r;
+    step = m.ell_height_aligned;
+    n = m.ell_num;
+}
+__device__ __forceinline__ void slot_row(const clspmv_sell_f32& m, long long r, size_t& at, int& step, int& n)
+{
+    const int sh = (int)m.sell_slice_height, sl = (int)r / sh, start = __ldg(m.sell_slice_ptr + sl);
+    at = (size_t)start + (r - (long long)sl * sh);
+    step = sh;
+    n = (__ldg(m.sell_slice_ptr + sl + 1) - start) / sh;
+}
+__device__ __forceinline__ const int* cols_of(const clspmv_ell_f32& m) { return m.ell_col_id; }
+__device__ __forceinline__ const int* cols_of(const clspmv_sell_f32& m) { return m.sell_col_id; }
+
+// SELL and 16-bit ELL rows of kSlotLoads slots and more: a group per row as in
+// the row walk, with the column ids, values and X rows of kSlotLoads slots in
+// flight together. The time follows the X loads in flight per SM: 8 a lane at
+// 32 warps. The row walk has 4 a lane at 64 warps for FP32 ELL, which keeps
+// it, but fewer for 16-bit values and one for SELL, whose slot count the
+// compiler does not see; short rows keep it too. Slots are summed in the same order.
+// B200, 27-point stencil of 101^3, us at k = 8 / 16 / 64: SELL 187 / 341 /
+// 1222 -> 94 / 170 / 612, ELL with BF16 values 123 / 225 / 822 -> 92 / 166 /
+// 595; SELL of the power law of 2^20 rows at k = 8 7.2 -> 2.1 ms.
+constexpr int kSlotLoads = 8;
+template <int VEC, class T, class M>
+__global__ void __launch_bounds__(kSpmmBlock, 4) k_spmm_slots(M m, const T* __restrict__ vals, Dense d)
+{
+    constexpr int U = kSlotLoads;
+    const int G = 1 << d.lshift;
+    const long long t = (long long)blockIdx.x * kSpmmBlock + threadIdx.x;
+    const int c0 = (int)(t & (G - 1)) * VEC;
+    if (c0 >= d.k) return;
+    const float* __restrict__ X = d.X + c0;
+    const long long groups = ((long long)gridDim.x * kSpmmBlock) >> d.lshift;
+    for (long long r = t >> d.lshift; r < m.matinfo.height; r += groups) {
+        size_t at;
+        int step, n;
+        slot_row(m, r, at, step, n);
+        const int* cp = cols_of(m) + at;
+        const T* vp = vals + at;
+        Acc<VEC> acc;
+        int i = 0;
+        auto batch = [&](auto count) {
+            constexpr int N = decltype(count)::value;
+            int c[N];
+            float v[N];
+            typename Acc<VEC>::X x[N];
+#pragma unroll
+            for (int u = 0; u < N; u++, cp += step, vp += step) {
+                c[u] = __ldg(cp);
+                v[u] = to_f(__ldg(vp));
+            }
+#pragma unroll
+            for (int u = 0; u < N; u++) x[u] = Acc<VEC>::load(X + (size_t)c[u] * d.ldx);
+#pragma unroll
+            for (int u = 0; u < N; u++) acc.fma_v(v[u], x[u]);
+            i += N;
+        };
+        while (i + U <= n) batch(std::integral_constant<int, U>{});
+        if (i + U / 2 <= n) batch(std::integral_constant<int, U / 2>{});
+        while (i < n) batch(std::integral_constant<int, 1>{});
+        acc.store(d.Y + (size_t)r * d.ldy + c0, d.scale ? d.alpha * d.scale[r] : d.alpha, d.beta);
+    }
+}
+
 // ---------------------------------------------------------------------------
 // Block walks: for_block(m, br, f) calls f(c4, base, s4, sh) for every stored
 // block of block row br. The block's first column is 4 * c4; the value of its
@@ -873,6 +941,21 @@ int launch_rows(const M& m, const void* vals, Dense d, int vec, cudaStream_t st)
     return after_launch(1);
 }
 
+// Slots per row that the host can tell: ELL's width; for SELL the mean, its slices hold at least that
+template <class T> inline bool long_slots(const clspmv_ell_f32& m) { return !std::is_same<T, float>::value && m.ell_num >= kSlotLoads; }
+template <class T> inline bool long_slots(const clspmv_sell_f32& m) { return (long long)m.matinfo.nnz >= (long long)kSlotLoads * m.matinfo.height; }
+
+template <class T, class M>
+int launch_slots(const M& m, const void* vals, Dense d, int vec, cudaStream_t st)
+{
+    if (!long_slots<T>(m)) return launch_rows<T>(m, vals, d, vec, st);
+    const int grid = grid_of((long long)m.matinfo.height << d.lshift);
+    const T* v = static_cast<const T*>(vals);
+    if (vec == 4) k_spmm_slots<4, T, M><<<grid, kSpmmBlock, 0, st>>>(m, v, d);
+    else k_spmm_slots<1, T, M><<<grid, kSpmmBlock, 0, st>>>(m, v, d);
+    return after_launch(1);
+}
+
 // CLSPMV_SPMM_BLOCK_ROWS=0 keeps the row walk for the block formats (measurements).
 bool block_rows_enabled()
 {
@@ -1020,15 +1103,15 @@ int spmm_typed(int format, const void* dev, const void* vals, Dense d, int vec, 
             return launch_chunks<T, false>(m.matinfo.height, m.matinfo.nnz, nullptr, m.coo_row_id, m.coo_col_id,
                                            vals ? vals : m.coo_data, d, vec, st);
         }
-#define ROWS(FMT, TYPE)                                                              \
+#define ROWS(FMT, TYPE, LAUNCH)                                                      \
     case FMT: {                                                                      \
         const auto& m = *static_cast<const TYPE*>(dev);                              \
-        return launch_rows<T>(m, vals ? vals : values_of(m), d, vec, st);            \
+        return LAUNCH<T>(m, vals ? vals : values_of(m), d, vec, st);                 \
     }
-        ROWS(CLSPMV_FORMAT_DIA, clspmv_dia_f32)
-        ROWS(CLSPMV_FORMAT_BDIA, clspmv_bdia_f32)
-        ROWS(CLSPMV_FORMAT_ELL, clspmv_ell_f32)
-        ROWS(CLSPMV_FORMAT_SELL, clspmv_sell_f32)
+        ROWS(CLSPMV_FORMAT_DIA, clspmv_dia_f32, launch_rows)
+        ROWS(CLSPMV_FORMAT_BDIA, clspmv_bdia_f32, launch_rows)
+        ROWS(CLSPMV_FORMAT_ELL, clspmv_ell_f32, launch_slots)
+        ROWS(CLSPMV_FORMAT_SELL, clspmv_sell_f32, launch_slots)
 #undef ROWS
 #define BLOCKS(FMT, TYPE)                                                            \
     case FMT: {                                                                      \
