@@ -782,9 +782,9 @@ __global__ void __launch_bounds__(kSpmmBlock, 4) k_spmm_runs(int rows, int nnz, 
                 XT xv[U];
 #pragma unroll
                 for (int u = 0; u < U; u++) {
-                    const int c = __shfl_sync(kWarpAll, cc[h + u], src, G);
-                    av[u] = __shfl_sync(kWarpAll, vv[h + u], src, G);
-                    rv[u] = __shfl_sync(kWarpAll, rr[h + u], src, G);
+                    const int c = G == 1 ? cc[h + u] : __shfl_sync(kWarpAll, cc[h + u], src, G);
+                    av[u] = G == 1 ? vv[h + u] : __shfl_sync(kWarpAll, vv[h + u], src, G);
+                    rv[u] = G == 1 ? rr[h + u] : __shfl_sync(kWarpAll, rr[h + u], src, G);
                     xv[u] = cols && rv[u] != kSegNoRow ? Acc<VEC>::load(X + (size_t)c * d.ldx) : Acc<VEC>::zero();
                 }
 #pragma unroll

@@ -215,11 +215,30 @@ def _torch_dtype(dt):
     return torch.float32 if dt == np.float32 else torch.int32
 
 
-def _stream_handle(stream) -> Optional[int]:
+def _bind_current_stream():
+    """The raw handle of torch's current stream on the current device.
+    torch.cuda.current_stream() builds a Stream object for it (3.2 us, more
+    than a kernel launch); the handle itself takes 0.1 us."""
     import torch
-    if stream is None:
-        stream = torch.cuda.current_stream()
-    return stream.cuda_stream
+    cuda, device, raw = torch.cuda, getattr(torch._C, "_cuda_getDevice", None), getattr(torch._C, "_cuda_getCurrentRawStream", None)
+
+    def current():
+        if raw is None or device is None or not cuda.is_initialized():
+            return cuda.current_stream().cuda_stream   # initialises CUDA, or raises as torch does
+        return raw(device())
+    return current
+
+
+_current_stream = None
+
+
+def _stream_handle(stream) -> Optional[int]:
+    if stream is not None:
+        return stream.cuda_stream
+    global _current_stream
+    if _current_stream is None:
+        _current_stream = _bind_current_stream()
+    return _current_stream()
 
 
 class DeviceMatrix:
@@ -303,8 +322,8 @@ class DeviceMatrix:
 
     def merge_plan(self, stream=None):
         """Tile coordinates for the merge-path CSR kernel (computed once)."""
-        import torch
         if self._plan is None:
+            import torch
             ntiles = lib().clspmv_csr_merge_tiles(self.shape[0], self.nnz)
             plan = torch.empty(2 * (ntiles + 1), dtype=torch.int32, device=self.tensors["csr_row_ptr"].device)
             check(lib().clspmv_csr_merge_plan(C.byref(self.struct), plan.data_ptr(), _stream_handle(stream)), "csr_merge_plan")
@@ -313,8 +332,8 @@ class DeviceMatrix:
 
     def chunk_plan(self, stream=None):
         """First row of every 256-nonzero chunk for the chunked CSR kernel (computed once)."""
-        import torch
         if getattr(self, "_chunk_plan", None) is None:
+            import torch
             n = lib().clspmv_csr_chunk_plan_size(self.nnz)
             plan = torch.empty(max(n, 1), dtype=torch.int32, device=self.tensors["csr_row_ptr"].device)
             check(lib().clspmv_csr_chunk_plan(C.byref(self.struct), plan.data_ptr(), _stream_handle(stream)), "csr_chunk_plan")
@@ -328,61 +347,56 @@ class DeviceMatrix:
         "chunk" (default; "merge" when col_id / data are not 16-byte aligned),
         "merge", "vector" or "scalar"; DIA / BDIA "bulk" stages the diagonals
         in shared memory by bulk copies; SELL "planned" reads only each
-        row's real entries (its length plan), which on B200 is slower than the
-        padded read for power-law slices: the tails of long rows are strided
-        column-major reads."""
-        L = lib()
+        row's real entries (its length plan)."""
         s = _stream_handle(stream)
-        _computable(self.fmt)
+        fmt = self.fmt
         if packed is not None:
-            if self.fmt == "csr" and variant == "chunk" and not ((self.struct.csr_col_id or 0) % 16
-                                                                 or packed.values.data_ptr() % 8):
-                check(L.clspmv_csr_chunk_spmv_packed(C.byref(self.struct), _abi.VALUE_TYPES[packed.value_type],
-                                                     packed.values.data_ptr(), packed.row_scale.data_ptr(),
-                                                     self.chunk_plan(stream).data_ptr(), x.data_ptr(), y.data_ptr(),
-                                                     alpha, beta, s), "csr_chunk_spmv_packed")
-                return
-            if self.fmt == "sell" and variant == "planned":
-                check(L.clspmv_sell_plan_spmv_packed(C.byref(self.struct), self.sell_plan(),
-                                                     _abi.VALUE_TYPES[packed.value_type], packed.values.data_ptr(),
-                                                     packed.row_scale.data_ptr(), x.data_ptr(), y.data_ptr(), alpha, beta,
-                                                     s), "sell_plan_spmv_packed")
-                return
-            plan = self.merge_plan(stream).data_ptr() if self.fmt == "csr" else None
-            check(L.clspmv_spmv_packed(_abi.FORMAT_IDS[self.fmt], C.byref(self.struct), _abi.VALUE_TYPES[packed.value_type],
-                                       packed.values.data_ptr(), packed.row_scale.data_ptr(), plan, x.data_ptr(),
-                                       y.data_ptr(), alpha, beta, s), "spmv_packed")
-            return
-        if self.fmt == "csr":
-            if variant == "merge":
-                plan = self.merge_plan(stream)
-                check(L.clspmv_csr_merge_spmv_f32(C.byref(self.struct), plan.data_ptr(), x.data_ptr(), y.data_ptr(),
-                                                  alpha, beta, s), "csr_merge_spmv")
-            elif variant == "chunk":
+            return self._spmv_packed(lib(), x, y, alpha, beta, stream, s, variant, packed)
+        struct, xp, yp = C.byref(self.struct), x.data_ptr(), y.data_ptr()
+        if fmt == "csr":
+            if variant == "chunk":
                 if (self.struct.csr_col_id or 0) % 16 or (self.struct.csr_data or 0) % 16:
                     return self.spmv(x, y, alpha, beta, stream, variant="merge")
-                plan = self.chunk_plan(stream)
-                check(L.clspmv_csr_chunk_spmv_f32(C.byref(self.struct), plan.data_ptr(), x.data_ptr(), y.data_ptr(),
-                                                  alpha, beta, s), "csr_chunk_spmv")
+                name, rc = "csr_chunk_spmv", lib().clspmv_csr_chunk_spmv_f32(struct, self.chunk_plan(stream).data_ptr(), xp, yp,
+                                                                             alpha, beta, s)
+            elif variant == "merge":
+                name, rc = "csr_merge_spmv", lib().clspmv_csr_merge_spmv_f32(struct, self.merge_plan(stream).data_ptr(), xp, yp,
+                                                                             alpha, beta, s)
             elif variant == "vector":
-                check(L.clspmv_csr_vector_spmv_f32(C.byref(self.struct), x.data_ptr(), y.data_ptr(), alpha, beta,
-                                                   threads_per_row, s), "csr_vector_spmv")
+                name, rc = "csr_vector_spmv", lib().clspmv_csr_vector_spmv_f32(struct, xp, yp, alpha, beta, threads_per_row, s)
             elif variant == "scalar":
-                check(L.clspmv_csr_scalar_spmv_f32(C.byref(self.struct), x.data_ptr(), y.data_ptr(), alpha, beta, s),
-                      "csr_scalar_spmv")
+                name, rc = "csr_scalar_spmv", lib().clspmv_csr_scalar_spmv_f32(struct, xp, yp, alpha, beta, s)
             else:
                 raise ValueError(variant)
+        elif fmt == "sell" and variant == "planned":
+            name, rc = "sell_plan_spmv", lib().clspmv_sell_plan_spmv_f32(struct, self.sell_plan(), xp, yp, alpha, beta, s)
+        else:
+            _computable(fmt)
+            name = f"clspmv_{fmt}_bulk_spmv_f32" if variant == "bulk" and fmt in ("dia", "bdia") else _SPMV[fmt]
+            rc = getattr(lib(), name)(struct, xp, yp, alpha, beta, s)
+        if rc:
+            check(rc, name)
+
+    def _spmv_packed(self, L, x, y, alpha, beta, stream, s, variant, packed) -> None:
+        """spmv from 16-bit values."""
+        _computable(self.fmt)
+        if self.fmt == "csr" and variant == "chunk" and not ((self.struct.csr_col_id or 0) % 16
+                                                             or packed.values.data_ptr() % 8):
+            check(L.clspmv_csr_chunk_spmv_packed(C.byref(self.struct), _abi.VALUE_TYPES[packed.value_type],
+                                                 packed.values.data_ptr(), packed.row_scale.data_ptr(),
+                                                 self.chunk_plan(stream).data_ptr(), x.data_ptr(), y.data_ptr(),
+                                                 alpha, beta, s), "csr_chunk_spmv_packed")
             return
         if self.fmt == "sell" and variant == "planned":
-            check(L.clspmv_sell_plan_spmv_f32(C.byref(self.struct), self.sell_plan(), x.data_ptr(), y.data_ptr(),
-                                              alpha, beta, s), "sell_plan_spmv")
+            check(L.clspmv_sell_plan_spmv_packed(C.byref(self.struct), self.sell_plan(),
+                                                 _abi.VALUE_TYPES[packed.value_type], packed.values.data_ptr(),
+                                                 packed.row_scale.data_ptr(), x.data_ptr(), y.data_ptr(), alpha, beta,
+                                                 s), "sell_plan_spmv_packed")
             return
-        if self.fmt in ("dia", "bdia") and variant == "bulk":
-            name = f"clspmv_{self.fmt}_bulk_spmv_f32"
-            check(getattr(L, name)(C.byref(self.struct), x.data_ptr(), y.data_ptr(), alpha, beta, s), name)
-            return
-        name = _SPMV[self.fmt]
-        check(getattr(L, name)(C.byref(self.struct), x.data_ptr(), y.data_ptr(), alpha, beta, s), name)
+        plan = self.merge_plan(stream).data_ptr() if self.fmt == "csr" else None
+        check(L.clspmv_spmv_packed(_abi.FORMAT_IDS[self.fmt], C.byref(self.struct), _abi.VALUE_TYPES[packed.value_type],
+                                   packed.values.data_ptr(), packed.row_scale.data_ptr(), plan, x.data_ptr(),
+                                   y.data_ptr(), alpha, beta, s), "spmv_packed")
 
     def pack(self, value_type: str = "bf16", stream=None) -> "PackedValues":
         """16-bit values ("bf16" or "f16") with per-row scales, for spmm."""
