@@ -393,6 +393,37 @@ __device__ __forceinline__ void sell_rows4_cta(const SellArgsT<V>& a, int cta, i
     }
 }
 
+// The same with each row's real length (rlen): a thread stops at the longest
+// of its 4 rows and a row at its own end, so padding adds nothing.
+template <bool ATOMIC, class V>
+__device__ __forceinline__ void sell_rows4_len_cta(const SellArgsT<V>& a, const int* __restrict__ rlen, int cta, int ncta)
+{
+    const uint64_t pe = policy_evict_first(), pl = policy_evict_last();
+    long long b, e;
+    cta_share(a.rows, 4, cta, ncta, b, e);
+    const int sh = a.slice_height;
+    for (long long row0 = b + threadIdx.x * 4; row0 < e; row0 += kBlock * 4) {
+        const int s = (int)(row0 / sh), lr = (int)(row0 - (long long)s * sh);
+        const size_t base = (size_t)a.slice_ptr[s] + lr;
+        int n[4];
+#pragma unroll
+        for (int i = 0; i < 4; i++) n[i] = row0 + i < a.rows ? __ldg(rlen + row0 + i) : 0;
+        const int most = max(max(n[0], n[1]), max(n[2], n[3]));
+        float acc[4] = {0.f, 0.f, 0.f, 0.f};
+#pragma unroll 4
+        for (int k = 0; k < most; k++) {
+            const int4 c = ld_stream_i4(a.col + base + (size_t)k * sh, pe);
+            const float4 v = ldv4(a.data + base + (size_t)k * sh, pe);
+            const float x0 = ld_x(a.x + c.x, pl), x1 = ld_x(a.x + c.y, pl), x2 = ld_x(a.x + c.z, pl), x3 = ld_x(a.x + c.w, pl);
+            if (k < n[0]) acc[0] = fmaf(v.x, x0, acc[0]);
+            if (k < n[1]) acc[1] = fmaf(v.y, x1, acc[1]);
+            if (k < n[2]) acc[2] = fmaf(v.z, x2, acc[2]);
+            if (k < n[3]) acc[3] = fmaf(v.w, x3, acc[3]);
+        }
+        y_put4<ATOMIC>(acc, row0, e, a.y, a.alpha, a.beta, scl(a));
+    }
+}
+
 // ---------------------------------------------------------------------------
 // SELL without its padding. The converter pads every row of a slice to the
 // slice's widest row with the row's previous column id and value 0
@@ -515,6 +546,20 @@ __device__ __forceinline__ void sell_tail_compact_cta(const SellArgsT<V>& a, con
     }
 }
 
+// Columns of a warp's runs in sell_masked_cta with FEW: kSellWarpCols, or
+// fewer (down to 4 warp steps of G columns) where that would leave warps
+// without a run: a matrix of 2,000 rows of 31 has 1,953 columns, 31 runs of
+// 64 but 123 of 16. Split walk on B200, rows of 31 at 2k / 20k rows 16 / 18 ->
+// 9 / 10 us, power law 16 / 22 -> 10 / 13. The walk of a matrix of many columns
+// keeps the run a constant: as a variable it spills one more of its 32
+// registers (uneven rows of 20 at 200k rows 29.8 -> 31.1 us).
+template <int G>
+__device__ __forceinline__ int sell_run(long long total_cols, long long nwarps)
+{
+    const long long share = (total_cols + nwarps - 1) / nwarps;
+    return (int)min((long long)kSellWarpCols, max(4LL * G, (share + 4 * G - 1) / (4 * G) * (4 * G)));
+}
+
 // SELL with the padding skipped, on the column-balanced mapping of sell_cta:
 // the Q lanes of a column each own 4 rows of the slice, and a lane issues its
 // 128-bit loads only for the columns before the longest real length of its 4
@@ -529,7 +574,7 @@ __device__ __forceinline__ void sell_tail_compact_cta(const SellArgsT<V>& a, con
 // only the first head[s+1] - head[s] columns of slice s are walked: the
 // columns up to its second-longest row, the rest of its longest row being
 // left to sell_tail_cta.
-template <int Q, bool ATOMIC_ALL, class V = float>
+template <int Q, bool ATOMIC_ALL, bool FEW, class V = float>
 __device__ __forceinline__ void sell_masked_cta(const SellArgsT<V>& a, const int* __restrict__ rlen, int cta, int ncta,
                                                 const int* __restrict__ head = nullptr)
 {
@@ -543,8 +588,9 @@ __device__ __forceinline__ void sell_masked_cta(const SellArgsT<V>& a, const int
     const int g = lane / Q, q = lane % Q;
     const long long nwarps_total = (long long)ncta * (kBlock / 32);
     const long long wid = (long long)cta * (kBlock / 32) + (threadIdx.x >> 5);
-    for (long long c0 = wid * kSellWarpCols; c0 < total_cols; c0 += nwarps_total * kSellWarpCols) {
-        const long long c1 = min(c0 + kSellWarpCols, total_cols);
+    const int run = FEW ? sell_run<G>(total_cols, nwarps_total) : kSellWarpCols;
+    for (long long c0 = wid * run; c0 < total_cols; c0 += nwarps_total * run) {
+        const long long c1 = min(c0 + run, total_cols);
         int lo = 0, hi = a.nslice - 1;
         while (lo < hi) {
             const int mid = (lo + hi) >> 1;

@@ -103,6 +103,12 @@ __global__ void __launch_bounds__(kBlock) k_sell_rows(SellArgsT<V> a) { sell_row
 template <bool A, class V>
 __global__ void __launch_bounds__(kBlock) k_sell_rows4(SellArgsT<V> a) { sell_rows4_cta<A>(a, blockIdx.x, gridDim.x, nullptr); }
 
+template <bool A, class V>
+__global__ void __launch_bounds__(kBlock) k_sell_rows4_len(SellArgsT<V> a, const int* __restrict__ rlen)
+{
+    sell_rows4_len_cta<A>(a, rlen, blockIdx.x, gridDim.x);
+}
+
 __global__ void __launch_bounds__(kBlock) k_sell_rlen(const int* __restrict__ slice_ptr, const int* __restrict__ col,
                                                       const float* __restrict__ data, int sh, long long rows, int* rlen)
 {
@@ -114,11 +120,11 @@ __global__ void __launch_bounds__(kBlock) k_sell_rlen(const int* __restrict__ sl
 // power-law SELL-32 heads, 0.273 ms for the planned SpMV against 0.292 at 6
 // CTAs (40 registers) and 0.318 at 4 (62 registers): the walk is latency
 // bound, so warps in flight count more than the spills
-template <int Q, bool A, class V = float>
+template <int Q, bool A, bool FEW, class V = float>
 __global__ void __launch_bounds__(kBlock, 8) k_sell_masked(SellArgsT<V> a, const int* __restrict__ rlen,
                                                            const int* __restrict__ head)
 {
-    sell_masked_cta<Q, A, V>(a, rlen, blockIdx.x, gridDim.x, head);
+    sell_masked_cta<Q, A, FEW, V>(a, rlen, blockIdx.x, gridDim.x, head);
 }
 template <bool A>
 __global__ void __launch_bounds__(kBlock) k_sell_head(SellArgs a, const int* __restrict__ rlen)
@@ -145,7 +151,7 @@ __global__ void __launch_bounds__(kBlock) k_sell_tail_compact(SellArgsT<V> a, co
 // CTA may add to the same row meanwhile), so the latency-bound head walk and
 // the bandwidth-bound tails share the SMs instead of running one after the
 // other.
-template <int Q, class V>
+template <int Q, bool FEW, class V>
 __global__ void __launch_bounds__(kBlock, 8) k_sell_planned_one(SellArgsT<V> a, const int* __restrict__ rlen,
                                                                 const int* __restrict__ head, const int2* __restrict__ items,
                                                                 const int* __restrict__ tail_off,
@@ -154,7 +160,7 @@ __global__ void __launch_bounds__(kBlock, 8) k_sell_planned_one(SellArgsT<V> a, 
     if ((int)blockIdx.x < ntail)
         sell_tail_compact_cta<V>(a, rlen, items, tail_off, tail_col, nitems, blockIdx.x, ntail);
     else
-        sell_masked_cta<Q, true, V>(a, rlen, blockIdx.x - ntail, gridDim.x - ntail, head);
+        sell_masked_cta<Q, true, FEW, V>(a, rlen, blockIdx.x - ntail, gridDim.x - ntail, head);
 }
 
 // Share of the one launch's CTAs on the tails, per mille: measured on B200
@@ -541,12 +547,12 @@ int launch_sell(const clspmv_sell_f32* m, const float* x, float* y, float alpha,
 // by sell_one_permille, but no more than the tail items keep busy (a CTA
 // walks 8 items at a time).
 template <class V>
-int launch_sell_one(const SellArgsT<V>& a, int sh, const int* rlen, const int* head, const int2* split_items,
+int launch_sell_one(const SellArgsT<V>& a, int sh, bool few, const int* rlen, const int* head, const int2* split_items,
                     long long nsplit, const int* tail_off, const int* tail_col, cudaStream_t st)
 {
     return dispatch_lanes(sh / 4, [&](auto q) {
         constexpr int Q = decltype(q)::value;
-        auto k = k_sell_planned_one<Q, V>;
+        auto k = few ? k_sell_planned_one<Q, true, V> : k_sell_planned_one<Q, false, V>;
         const unsigned grid = persistent_grid(k, 1LL << 40, 1);
         long long ntail = (long long)grid * sell_one_permille() / 1000;
         ntail = std::min(ntail, (nsplit + kBlock / 32 - 1) / (kBlock / 32));
@@ -564,7 +570,7 @@ int launch_sell_one(const SellArgsT<V>& a, int sh, const int* rlen, const int* h
 // kSellTailCols entries (split_items); with the tails' compact column ids
 // both run in one launch (launch_sell_one). Other slice heights: each row's
 // first kSellHead entries with a thread per row, then the tails (items).
-int launch_sell_planned(const clspmv_sell_f32* m, const int* rlen, const int2* items, long long nitems, const int* head,
+int launch_sell_planned(const clspmv_sell_f32* m, bool few, const int* rlen, const int2* items, long long nitems, const int* head,
                         const int2* split_items, long long nsplit, const int* tail_off, const int* tail_col,
                         const float* x, float* y, float alpha, float beta, cudaStream_t st, bool atomic)
 {
@@ -583,11 +589,12 @@ int launch_sell_planned(const clspmv_sell_f32* m, const int* rlen, const int2* i
         }
         a.beta = 1.0f;
         if (head && tail_col && nsplit > 0 && sell_one_permille() > 0)
-            return launch_sell_one<float>(a, sh, rlen, head, split_items, nsplit, tail_off, tail_col, st);
+            return launch_sell_one<float>(a, sh, few, rlen, head, split_items, nsplit, tail_off, tail_col, st);
         int rc = dispatch_lanes(sh / 4, [&](auto q) {
             constexpr int Q = decltype(q)::value;
-            if (atomic) k_sell_masked<Q, true><<<persistent_grid(k_sell_masked<Q, true>, 1LL << 40, 1), kBlock, 0, st>>>(a, rlen, head);
-            else k_sell_masked<Q, false><<<persistent_grid(k_sell_masked<Q, false>, 1LL << 40, 1), kBlock, 0, st>>>(a, rlen, head);
+            auto k = atomic ? (few ? k_sell_masked<Q, true, true> : k_sell_masked<Q, true, false>)
+                            : (few ? k_sell_masked<Q, false, true> : k_sell_masked<Q, false, false>);
+            k<<<persistent_grid(k, 1LL << 40, 1), kBlock, 0, st>>>(a, rlen, head);
             return after_launch(1);
         });
         if (rc || !head || nsplit == 0) return rc;
@@ -609,7 +616,7 @@ int launch_sell_planned(const clspmv_sell_f32* m, const int* rlen, const int2* i
 // The planned walk with 16-bit values (per-row scales): slice heights
 // 4..128 with the heads / compact tails split; otherwise the padded read.
 template <class V>
-int launch_sell_planned_packed(const clspmv_sell_f32* m, const V* data, const float* scale, const int* rlen, const int* head,
+int launch_sell_planned_packed(const clspmv_sell_f32* m, bool few, const V* data, const float* scale, const int* rlen, const int* head,
                                const int2* split_items, long long nsplit, const int* tail_off, const int* tail_col,
                                const float* x, float* y, float alpha, float beta, cudaStream_t st)
 {
@@ -624,10 +631,11 @@ int launch_sell_planned_packed(const clspmv_sell_f32* m, const V* data, const fl
     int rc = prescale(y, rows, beta, st);
     if (rc) return rc;
     if (nsplit > 0 && sell_one_permille() > 0)
-        return launch_sell_one<V>(a, sh, rlen, head, split_items, nsplit, tail_off, tail_col, st);
+        return launch_sell_one<V>(a, sh, few, rlen, head, split_items, nsplit, tail_off, tail_col, st);
     rc = dispatch_lanes(sh / 4, [&](auto q) {
         constexpr int Q = decltype(q)::value;
-        k_sell_masked<Q, false, V><<<persistent_grid(k_sell_masked<Q, false, V>, 1LL << 40, 1), kBlock, 0, st>>>(a, rlen, head);
+        auto k = few ? k_sell_masked<Q, false, true, V> : k_sell_masked<Q, false, false, V>;
+        k<<<persistent_grid(k, 1LL << 40, 1), kBlock, 0, st>>>(a, rlen, head);
         return after_launch(1);
     });
     if (rc || nsplit == 0) return rc;
@@ -1031,6 +1039,8 @@ struct clspmv_sell_plan {
     long long rows = 0, nitems = 0, nsplit = 0, entries = 0;
     long long sector_bytes = 0;   // col + data bytes of the 32-byte sectors holding real entries
     long long line_bytes = 0;     // bytes the split walk must read in 128-byte lines (see clspmv_sell_plan_line_bytes)
+    bool few = false;          // columns for fewer than a quarter of the device's warps' whole runs (sell_run)
+    int even = 0;              // little padding and at most this many columns on average (12 or 32), 0: else
     bool split = true;         // walk the heads and the tails apart (power-of-two slice heights)
     bool compact = true;       // the tails' column ids from tail_col
 };
@@ -1074,6 +1084,7 @@ int clspmv_sell_plan_create(const clspmv_sell_f32* m, clspmv_sell_plan** out)
             for (int k = l2; arg >= 0 && k < l1; k += kSellTailCols) split.push_back(make_int2((int)arg, k));
         }
         p->nsplit = (long long)split.size();
+        p->few = head[(size_t)ns] < 148 * 64 * kSellWarpCols / 4;
         rc = cuda_status(cudaMalloc(&p->head, sizeof(int) * head.size()));
         if (!rc) rc = cuda_status(cudaMemcpy(p->head, head.data(), sizeof(int) * head.size(), cudaMemcpyHostToDevice));
         if (!rc) rc = cuda_status(cudaMalloc(&p->split_items, sizeof(int2) * std::max<size_t>(1, split.size())));
@@ -1121,6 +1132,9 @@ int clspmv_sell_plan_create(const clspmv_sell_f32* m, clspmv_sell_plan** out)
             for (uint64_t w : dline) lines += __builtin_popcountll(w);
             for (uint64_t w : cline) lines += __builtin_popcountll(w);
             p->line_bytes = 128 * lines + 4 * tail_entries + 4 * rows + 4 * (ns + 1) + 12 * (long long)split.size() + 4;
+            const long long slots = sp[(size_t)ns];
+            if (shs % 4 == 0 && ns * shs >= rows && 4 * p->line_bytes >= 3 * 8 * slots)
+                p->even = slots <= 12 * ns * shs ? 12 : slots <= 32 * ns * shs ? 32 : 0;
         }
         // CLSPMV_SELL_SPLIT=0 walks every column instead, CLSPMV_SELL_TAIL_COMPACT=0
         // reads the tails' column ids in place (for measurements)
@@ -1154,6 +1168,36 @@ int clspmv_sell_plan_create(const clspmv_sell_f32* m, clspmv_sell_plan** out)
 
 }  // extern "C"
 
+namespace {
+// 4 rows per thread up to their real lengths, for plans marked even.
+template <class V>
+int launch_sell_even(const clspmv_sell_f32* m, const V* data, const float* scale, const int* rlen, const float* x, float* y,
+                     float alpha, float beta, cudaStream_t st, bool atomic)
+{
+    const int rows = m->matinfo.height;
+    if (rows <= 0) return CLSPMV_OK;
+    SellArgsT<V> a{rows, (int)m->sell_slice_height, m->sell_slice_num, m->sell_slice_ptr, m->sell_col_id, data, x, y, alpha,
+                   beta, scale};
+    if (atomic) k_sell_rows4_len<true, V><<<persistent_grid(k_sell_rows4_len<true, V>, rows, kBlock * 4), kBlock, 0, st>>>(a, rlen);
+    else k_sell_rows4_len<false, V><<<persistent_grid(k_sell_rows4_len<false, V>, rows, kBlock * 4), kBlock, 0, st>>>(a, rlen);
+    return after_launch(1);
+}
+// Nearly every line holds entries (on the power law 0.6 of them) and rows are
+// short: nothing for the split walk to save, and 4 rows per thread need no
+// scaled y, no atomics and no shuffles. Measured on B200 (us, split walk -> 4
+// rows per thread): 5-point Laplacian of 2k / 200k / 1M rows 30 / 28 / 41 ->
+// 3.6 / 4.6 / 10.5, rows of 9 with BF16 values at 1M 39 -> 21; 1M rows of 27
+// 64 -> 56, of 10 to 30 at random 117 -> 99. Rows of 13 to 32 in smaller matrices leave
+// the thread's walk too few threads (2k rows of 31: 10.2 us against 6.8 for
+// runs of columns), and with 16-bit values it is the slower one (1M of 27: 53 -> 62).
+template <class V>
+bool takes_even(const clspmv_sell_f32* m, const clspmv_sell_plan* p, const V* data, const float* x, const float* y)
+{
+    if (!p->even || !m || !x || !y || !m->sell_slice_ptr || !data || !aligned16(m->sell_col_id) || !aligned_v4(data)) return false;
+    return p->even == 12 || (std::is_same<V, float>::value && m->matinfo.height >= 500000);
+}
+}  // namespace
+
 namespace clspmv {
 // The planned walk for a caller that already applied beta and adds into y
 // with the other parts of a Cocktail matrix (atomic = true).
@@ -1161,7 +1205,9 @@ int launch_sell_plan(const clspmv_sell_f32* m, const clspmv_sell_plan* p, const 
                      cudaStream_t st, bool atomic)
 {
     if (!p) return CLSPMV_ERR_ARG;
-    return launch_sell_planned(m, p->rlen, p->items, p->nitems, p->split ? p->head : nullptr, p->split_items, p->nsplit,
+    if (m && takes_even(m, p, m->sell_data, x, y))
+        return launch_sell_even<float>(m, m->sell_data, nullptr, p->rlen, x, y, alpha, beta, st, atomic);
+    return launch_sell_planned(m, p->few, p->rlen, p->items, p->nitems, p->split ? p->head : nullptr, p->split_items, p->nsplit,
                                p->tail_off, p->compact ? p->tail_col : nullptr, x, y, alpha, beta, st, atomic);
 }
 }  // namespace clspmv
@@ -1171,9 +1217,7 @@ extern "C" {
 int clspmv_sell_plan_spmv_f32(const clspmv_sell_f32* m, const clspmv_sell_plan* p, const float* x, float* y, float alpha,
                               float beta, clspmv_stream_t s)
 {
-    if (!p) return CLSPMV_ERR_ARG;
-    return launch_sell_planned(m, p->rlen, p->items, p->nitems, p->split ? p->head : nullptr, p->split_items, p->nsplit,
-                               p->tail_off, p->compact ? p->tail_col : nullptr, x, y, alpha, beta, S(s), false);
+    return launch_sell_plan(m, p, x, y, alpha, beta, S(s), false);
 }
 
 int clspmv_sell_plan_spmv_packed(const clspmv_sell_f32* m, const clspmv_sell_plan* p, int value_type, const void* values,
@@ -1182,11 +1226,15 @@ int clspmv_sell_plan_spmv_packed(const clspmv_sell_f32* m, const clspmv_sell_pla
     if (!p) return CLSPMV_ERR_ARG;
     const int* head = p->split ? p->head : nullptr;
     const int* tc = p->compact ? p->tail_col : nullptr;
+    if (row_scale && value_type == CLSPMV_VALUES_BF16 && takes_even(m, p, static_cast<const __nv_bfloat16*>(values), x, y))
+        return launch_sell_even(m, static_cast<const __nv_bfloat16*>(values), row_scale, p->rlen, x, y, alpha, beta, S(s), false);
+    if (row_scale && value_type == CLSPMV_VALUES_F16 && takes_even(m, p, static_cast<const __half*>(values), x, y))
+        return launch_sell_even(m, static_cast<const __half*>(values), row_scale, p->rlen, x, y, alpha, beta, S(s), false);
     if (value_type == CLSPMV_VALUES_BF16)
-        return launch_sell_planned_packed(m, static_cast<const __nv_bfloat16*>(values), row_scale, p->rlen, head,
+        return launch_sell_planned_packed(m, p->few, static_cast<const __nv_bfloat16*>(values), row_scale, p->rlen, head,
                                           p->split_items, p->nsplit, p->tail_off, tc, x, y, alpha, beta, S(s));
     if (value_type == CLSPMV_VALUES_F16)
-        return launch_sell_planned_packed(m, static_cast<const __half*>(values), row_scale, p->rlen, head, p->split_items,
+        return launch_sell_planned_packed(m, p->few, static_cast<const __half*>(values), row_scale, p->rlen, head, p->split_items,
                                           p->nsplit, p->tail_off, tc, x, y, alpha, beta, S(s));
     return CLSPMV_ERR_ARG;
 }
