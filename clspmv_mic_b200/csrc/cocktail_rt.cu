@@ -118,14 +118,31 @@ void release(clspmv_cocktail_handle* h)
     if (h->cap) cudaStreamDestroy(h->cap);
 }
 
-constexpr int kIterUnroll = 16;   // steps per replayed graph
+constexpr int kIterUnroll = 16;   // steps per replayed graph (even: see iterate_steps)
+
+// With beta = 0 a step reads nothing but the last result, which x and y both
+// hold: the steps may go back and forth between the two buffers, without the
+// copy that is 2 of a step's 5 us on a matrix that stays in L2. y must then
+// serve as a vector of the matrix: as long, and aligned like x.
+bool back_and_forth(const clspmv_cocktail_handle* h, const float* x, const float* y, float beta)
+{
+    return beta == 0.0f && h->dev.mat_width == h->dev.mat_height && ((reinterpret_cast<uintptr_t>(x) | reinterpret_cast<uintptr_t>(y)) & 15u) == 0;
+}
 
 // n steps of the reference's loop (src/eval.cpp:44-50): y <- alpha*A*x + beta*y,
 // then the first mat_height entries of x <- y (cpy_vector_from_gpu,
 // src/spmv_cocktail.cpp:1510-1556), stream ordered, no host synchronisation.
+// Back and forth, the result of n steps is in x alone (n even) or y alone (odd).
 int iterate_steps(clspmv_cocktail_handle* h, float* x, float* y, float alpha, float beta, int n, cudaStream_t st)
 {
     const size_t bytes = sizeof(float) * (size_t)h->dev.mat_height;
+    if (back_and_forth(h, x, y, beta)) {
+        for (int i = 0; i < n; i++) {
+            const int rc = clspmv_cocktail_spmv_f32(h, i % 2 ? y : x, i % 2 ? x : y, alpha, 0.0f, st);
+            if (rc) return rc;
+        }
+        return CLSPMV_OK;
+    }
     for (int i = 0; i < n; i++) {
         int rc = clspmv_cocktail_spmv_f32(h, x, y, alpha, beta, st);
         if (!rc && bytes) rc = cuda_status(cudaMemcpyAsync(x, y, bytes, cudaMemcpyDeviceToDevice, st));
@@ -279,6 +296,9 @@ int clspmv_cocktail_iterate_f32(clspmv_cocktail_handle* h, float* x, float* y, f
         if (!rc) rc = after_launch(0);
     }
     if (!rc) rc = iterate_steps(h, x, y, alpha, beta, rest, st);
+    const size_t bytes = sizeof(float) * (size_t)h->dev.mat_height;
+    if (!rc && iterations > 0 && bytes && back_and_forth(h, x, y, beta))   // the whole graphs ended in x
+        rc = cuda_status(cudaMemcpyAsync(rest % 2 ? x : y, rest % 2 ? y : x, bytes, cudaMemcpyDeviceToDevice, st));
     return rc;
 }
 
