@@ -26,6 +26,8 @@ struct clspmv_cocktail_handle {
     clspmv_cocktail_f32 dev;          // part structs with device pointers
     int* chunk_plan = nullptr;        // first row of every nonzero chunk of the CSR part
     int nparts = 0;
+    int bdia_ndiag = 0;               // diagonals of the BDIA part
+    ResidentRows rows;                // how a lone COO / CSR part fits a cluster
     FusedPlan* fused = nullptr;       // one persistent launch over all parts (two or more parts)
     clspmv_sell_plan* sell_plan = nullptr;   // the SELL part's length plan, when it reads well under the stored slots
     int schedule = CLSPMV_SCHEDULE_AUTO;
@@ -151,6 +153,26 @@ int iterate_steps(clspmv_cocktail_handle* h, float* x, float* y, float alpha, fl
     return CLSPMV_OK;
 }
 
+// Steps from which the one launch that loads the matrix into a cluster pays.
+constexpr int kResidentSteps = 4;
+
+// The steps in one launch, for a matrix of one DIA, BDIA, COO or CSR part
+// that fits a cluster's shared memory; CLSPMV_ERR_UNSUPPORTED otherwise.
+int resident_steps(clspmv_cocktail_handle* h, float* x, float* y, float alpha, float beta, int steps, cudaStream_t st)
+{
+    const clspmv_cocktail_f32& d = h->dev;
+    if (h->nparts != 1 || steps < kResidentSteps) return CLSPMV_ERR_UNSUPPORTED;
+    if (d.ifusedia && d.dia.matinfo.height == d.mat_height && d.mat_height <= d.dia.dia_length_aligned &&
+        resident_iterate_fits(d.mat_height, d.dia.dia_num))
+        return resident_iterate_dia(&d.dia, x, y, alpha, beta, steps, st);
+    if (d.ifusebdia && d.bdia.matinfo.height == d.mat_height && d.mat_height <= d.bdia.bdia_length_aligned &&
+        resident_iterate_fits(d.mat_height, h->bdia_ndiag))
+        return resident_iterate_bdia(&d.bdia, h->bdia_ndiag, x, y, alpha, beta, steps, st);
+    if (d.ifusecoo && h->rows.ctas) return resident_iterate_coo(&d.coo, h->rows, x, y, alpha, beta, steps, st);
+    if (d.ifusecsr && h->rows.ctas && h->csr_lanes == 0) return resident_iterate_csr(&d.csr, h->rows, x, y, alpha, beta, steps, st);
+    return CLSPMV_ERR_UNSUPPORTED;
+}
+
 int iteration_graph(clspmv_cocktail_handle* h, float* x, float* y, float alpha, float beta)
 {
     if (h->iter_exec && h->iter_x == x && h->iter_y == y && h->iter_alpha == alpha && h->iter_beta == beta)
@@ -216,6 +238,7 @@ int clspmv_cocktail_upload_f32(const clspmv_cocktail_f32* host, clspmv_cocktail_
     UP(ifusecsr, csr, clspmv_upload_csr_f32)
     UP(ifusecoo, coo, clspmv_upload_coo_f32)
 #undef UP
+    if (d.ifusebdia && c.bdia.bdia_band_num > 0) h->bdia_ndiag = c.bdia.bdia_bptr[c.bdia.bdia_band_num];
     if (!rc && d.ifusesell && !sell_plan_disabled()) {
         // SELL parts of uneven rows (slices padded to their longest row) take
         // the padding-free walk when its lines come to under 3/4 of the slots
@@ -238,6 +261,10 @@ int clspmv_cocktail_upload_f32(const clspmv_cocktail_f32* host, clspmv_cocktail_
         h->nparts++;
         rc = cuda_status(cudaStreamCreateWithFlags(&h->streams[p], cudaStreamNonBlocking));
         if (!rc) rc = cuda_status(cudaEventCreateWithFlags(&h->join[p], cudaEventDisableTiming));
+    }
+    if (!rc && h->nparts == 1) {
+        if (d.ifusecoo && d.coo.matinfo.height == d.mat_height) h->rows = resident_rows_plan(d.mat_height, c.coo.matinfo.nnz, c.coo.coo_row_id, nullptr);
+        if (d.ifusecsr && d.csr.matinfo.height == d.mat_height) h->rows = resident_rows_plan(d.mat_height, c.csr.matinfo.nnz, nullptr, c.csr.csr_row_ptr);
     }
     if (!rc) rc = cuda_status(cudaEventCreateWithFlags(&h->fork, cudaEventDisableTiming));
     if (!rc && h->nparts >= 2) {
@@ -288,6 +315,10 @@ int clspmv_cocktail_iterate_f32(clspmv_cocktail_handle* h, float* x, float* y, f
     if (!h || !x || !y || x == y || iterations < 0) return CLSPMV_ERR_ARG;
     if (h->dev.mat_width < h->dev.mat_height) return CLSPMV_ERR_ARG;   // x must hold a copy of y
     cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);
+    {
+        const int rc = resident_steps(h, x, y, alpha, beta, iterations, st);
+        if (rc != CLSPMV_ERR_UNSUPPORTED) return rc;
+    }
     const int full = iterations / kIterUnroll, rest = iterations % kIterUnroll;
     int rc = CLSPMV_OK;
     if (full > 0) {
