@@ -698,8 +698,12 @@ int clspmv_cocktail_set_csr_lanes(clspmv_cocktail_handle* h, int lanes);
  * `iterations` times y <- alpha*A*x + beta*y, then the first mat_height
  * entries of x <- y (cpy_vector_from_gpu, src/spmv_cocktail.cpp:1510-1556).
  * Stream ordered with no host synchronisation (the reference waits after
- * every step): whole groups of 16 steps replay one CUDA graph captured once
- * per (x, y, alpha, beta) and cached in the handle, the rest launch directly.
+ * every step): from 4 steps on, one DIA, BDIA, COO or CSR part whose rows fit
+ * is held by the shared memory of one thread-block cluster and takes one
+ * launch; otherwise whole groups of 16 steps replay one CUDA graph captured
+ * once per (x, y, alpha, beta) and cached in the handle, the rest launch
+ * directly, and with beta = 0 on a square matrix the steps go back and forth
+ * between x and y in place of the copies.
  * Requires mat_width >= mat_height and x != y. alpha = beta = 1 is the
  * reference's loop. */
 int clspmv_cocktail_iterate_f32(clspmv_cocktail_handle* h, float* x, float* y, float alpha, float beta, int iterations,
