@@ -15,8 +15,10 @@
 // 183 GB) in kKeptMost arrays, the oldest leaving first; it is given back
 // when an allocation fails, when less than 1/8 of the device is left after
 // a large new one, and by clspmv_device_trim. Only arrays that device_alloc made
-// (and that the driver still reports with that size) are kept; any other
-// pointer goes to cudaFree.
+// are kept; any other pointer goes to cudaFree. An array is known by the
+// driver's id of its allocation, which no other one of the process gets: one
+// that the caller freed, or that a device reset took away, is neither handed
+// out nor freed again, whoever owns its address by then.
 #include <cuda.h>
 #include <algorithm>
 #include <list>
@@ -32,12 +34,17 @@ struct Kept {
     void* p;
     size_t bytes;
     int device;
+    unsigned long long id;
+};
+struct Made {
+    size_t bytes;
+    unsigned long long id;
 };
 
 std::mutex g_mu;
 std::list<Kept> g_kept;                              // oldest first
 std::unordered_map<int, size_t> g_kept_bytes;        // per device
-std::unordered_map<void*, size_t> g_made;            // arrays made by device_alloc and not yet cudaFree'd
+std::unordered_map<void*, Made> g_made;              // arrays made by device_alloc and not yet cudaFree'd
 
 constexpr size_t kGrain = 512;
 constexpr size_t kLarge = 64u << 20;
@@ -62,24 +69,36 @@ size_t limit_of(int device)
     return cache[device] = total / 64;
 }
 
-// Size the driver reports for the allocation that starts at p, 0 if p is no start of one.
-size_t driver_size(void* p)
+// The driver's id of the allocation at p, 0 if there is none (0.14 us).
+unsigned long long allocation_id(void* p)
 {
-    typedef CUresult (*Range)(CUdeviceptr*, size_t*, CUdeviceptr);
-    static const Range range = [] {
+    typedef CUresult (*Attribute)(void*, CUpointer_attribute, CUdeviceptr);
+    static const Attribute attribute = [] {
         void* fn = nullptr;
         cudaDriverEntryPointQueryResult q;
-        if (cudaGetDriverEntryPoint("cuMemGetAddressRange", &fn, cudaEnableDefault, &q) != cudaSuccess ||
+        if (cudaGetDriverEntryPoint("cuPointerGetAttribute", &fn, cudaEnableDefault, &q) != cudaSuccess ||
             q != cudaDriverEntryPointSuccess) {
             cudaGetLastError();
             fn = nullptr;
         }
-        return reinterpret_cast<Range>(fn);
+        return reinterpret_cast<Attribute>(fn);
     }();
-    CUdeviceptr base = 0;
-    size_t bytes = 0;
-    if (!range || range(&base, &bytes, reinterpret_cast<CUdeviceptr>(p)) != CUDA_SUCCESS) return 0;
-    return base == reinterpret_cast<CUdeviceptr>(p) ? bytes : 0;
+    unsigned long long id = 0;
+    if (!attribute || attribute(&id, CU_POINTER_ATTRIBUTE_BUFFER_ID, reinterpret_cast<CUdeviceptr>(p)) != CUDA_SUCCESS) return 0;
+    return id;
+}
+
+bool alive(const Kept& k) { return allocation_id(k.p) == k.id; }
+
+// Takes an entry off the list (g_mu held), and off the arrays made unless it is handed out.
+std::list<Kept>::iterator unlist(std::list<Kept>::iterator it, bool handed_out)
+{
+    g_kept_bytes[it->device] -= it->bytes;
+    if (!handed_out) {
+        auto made = g_made.find(it->p);
+        if (made != g_made.end() && made->second.id == it->id) g_made.erase(made);
+    }
+    return g_kept.erase(it);
 }
 
 // Takes the kept arrays of `device` (all devices: -1) off the list.
@@ -88,13 +107,12 @@ std::list<Kept> take_kept(int device)
     std::list<Kept> out;
     std::lock_guard<std::mutex> lock(g_mu);
     for (auto it = g_kept.begin(); it != g_kept.end();) {
-        auto next = std::next(it);
-        if (device < 0 || it->device == device) {
-            g_kept_bytes[it->device] -= it->bytes;
-            g_made.erase(it->p);
-            out.splice(out.end(), g_kept, it);
+        if (device >= 0 && it->device != device) {
+            ++it;
+            continue;
         }
-        it = next;
+        out.push_back(*it);
+        it = unlist(it, false);
     }
     return out;
 }
@@ -102,7 +120,7 @@ std::list<Kept> take_kept(int device)
 void free_all(const std::list<Kept>& l)
 {
     for (const Kept& k : l)
-        if (cudaFree(k.p) != cudaSuccess) cudaGetLastError();
+        if (alive(k) && cudaFree(k.p) != cudaSuccess) cudaGetLastError();
 }
 
 }  // namespace
@@ -116,16 +134,17 @@ int device_alloc(void** out, size_t bytes)
     {
         // the smallest kept array that holds the request and is at most 1/8 larger
         std::lock_guard<std::mutex> lock(g_mu);
-        auto best = g_kept.end();
         const size_t most = bytes + bytes / 8 + kGrain;
-        for (auto it = g_kept.begin(); it != g_kept.end(); ++it)
-            if (it->device == device && it->bytes >= bytes && it->bytes <= most && (best == g_kept.end() || it->bytes < best->bytes))
-                best = it;
-        if (best != g_kept.end()) {
-            *out = best->p;
-            g_kept_bytes[device] -= best->bytes;
-            g_kept.erase(best);
-            return CLSPMV_OK;
+        while (true) {
+            auto best = g_kept.end();
+            for (auto it = g_kept.begin(); it != g_kept.end(); ++it)
+                if (it->device == device && it->bytes >= bytes && it->bytes <= most && (best == g_kept.end() || it->bytes < best->bytes))
+                    best = it;
+            if (best == g_kept.end()) break;
+            const bool ok = alive(*best);
+            if (ok) *out = best->p;
+            unlist(best, ok);
+            if (ok) return CLSPMV_OK;
         }
     }
     void* p = nullptr;
@@ -139,7 +158,7 @@ int device_alloc(void** out, size_t bytes)
     }
     {
         std::lock_guard<std::mutex> lock(g_mu);
-        g_made[p] = bytes;
+        g_made[p] = Made{bytes, allocation_id(p)};
     }
     size_t fr = 0, total = 0;
     if (bytes >= kLarge && cudaMemGetInfo(&fr, &total) == cudaSuccess && fr < total / 8) free_all(take_kept(device));
@@ -150,18 +169,20 @@ int device_alloc(void** out, size_t bytes)
 void device_release(void* p, bool idle)
 {
     if (!p) return;
-    size_t bytes = 0;
+    Made made{0, 0};
+    const unsigned long long id = allocation_id(p);
     {
         std::lock_guard<std::mutex> lock(g_mu);
         for (const Kept& k : g_kept)
-            if (k.p == p) return;   // released already
+            if (k.p == p && k.id == id) return;   // released already
         auto it = g_made.find(p);
-        if (it != g_made.end()) bytes = it->second;
+        if (it != g_made.end() && it->second.id == id) made = it->second;
     }
+    const size_t bytes = made.bytes;
     cudaPointerAttributes at{};
-    bool keep = bytes && cudaPointerGetAttributes(&at, p) == cudaSuccess && at.type == cudaMemoryTypeDevice;
+    bool keep = id && bytes && cudaPointerGetAttributes(&at, p) == cudaSuccess && at.type == cudaMemoryTypeDevice;
     const size_t limit = keep ? limit_of(at.device) : 0;
-    if (keep) keep = bytes <= limit && driver_size(p) >= bytes;
+    if (keep) keep = bytes <= limit;
     int cur = -1;
     if (keep) {
         cudaGetDevice(&cur);
@@ -181,19 +202,24 @@ void device_release(void* p, bool idle)
     std::list<Kept> drop;
     {
         std::lock_guard<std::mutex> lock(g_mu);
-        for (const Kept& k : g_kept)
-            if (k.p == p) return;
-        g_kept.push_back(Kept{p, bytes, at.device});
+        for (auto it = g_kept.begin(); it != g_kept.end();) {
+            if (it->p != p) {
+                ++it;
+                continue;
+            }
+            if (it->id == id) return;
+            it = unlist(it, false);   // an array that is gone, whose address this one has
+        }
+        g_kept.push_back(Kept{p, bytes, at.device, id});
         size_t& held = g_kept_bytes[at.device];
         held += bytes;
         for (auto it = g_kept.begin(); (held > limit || g_kept.size() > kKeptMost) && it != g_kept.end();) {
-            auto next = std::next(it);
-            if (it->device == at.device) {
-                held -= it->bytes;
-                g_made.erase(it->p);
-                drop.splice(drop.end(), g_kept, it);
+            if (it->device != at.device) {
+                ++it;
+                continue;
             }
-            it = next;
+            drop.push_back(*it);
+            it = unlist(it, false);
         }
     }
     free_all(drop);

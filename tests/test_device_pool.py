@@ -1,0 +1,27 @@
+"""The list of kept device arrays (csrc/device_pool.cu), compiled against a
+stand-in for the CUDA calls it makes (compat/device_pool_check.cpp): no GPU.
+An array that a device reset took away or that the caller freed is not handed
+out and not freed again; the list's bounds and who leaves it hold."""
+import subprocess
+
+import pytest
+
+from conftest import ROOT
+
+
+@pytest.fixture(scope="module")
+def check(tmp_path_factory):
+    exe = tmp_path_factory.mktemp("pool") / "device_pool_check"
+    src = ROOT / "tests" / "compat" / "device_pool_check.cpp"
+    subprocess.run(["g++", "-std=c++17", "-g", "-fsanitize=address", f"-I{ROOT / 'include'}", f"-I{ROOT / 'clspmv_mic_b200' / 'csrc'}",
+                    "-I/usr/local/cuda/include", str(src), "-o", str(exe), "-lpthread"], check=True)
+
+    def run(name):
+        res = subprocess.run([str(exe), name], capture_output=True, text=True, timeout=60)
+        assert res.returncode == 0, res.stdout + res.stderr
+    return run
+
+
+@pytest.mark.parametrize("name", ["reuse", "bounds", "low_memory", "reset", "freed_by_the_caller"])
+def test_kept_arrays(check, name):
+    check(name)
