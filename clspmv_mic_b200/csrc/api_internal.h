@@ -10,9 +10,11 @@ int cuda_status(cudaError_t e);
 int after_launch(int n);
 
 // Device arrays that outlast a call, from the bounded list of released ones or cudaMalloc (device_pool.cu).
-// device_release waits for the device unless `idle` says that no work on the array is pending.
+// device_release waits for the array's device unless `idle_on` names it (or says kIdleAll): no work on the array is
+// pending there. It returns what the next array released with this one may name.
+constexpr int kIdleNone = -1, kIdleAll = -2;
 int device_alloc(void** out, size_t bytes);
-void device_release(void* p, bool idle);
+int device_release(void* p, int idle_on);
 
 // Format launchers (spmv_api.cu). With `atomic`, alpha*A*x is added into y
 // with red.global.add and beta is ignored (apply it first with

@@ -81,7 +81,8 @@ struct Allocs {
     {
         if (keep || ptrs.empty()) return;
         const bool idle = cudaStreamSynchronize(st) == cudaSuccess;   // the arrays were used on `st` alone
-        for (void* p : ptrs) clspmv::device_release(p, idle);
+        int idle_on = idle ? clspmv::kIdleAll : clspmv::kIdleNone;
+        for (void* p : ptrs) idle_on = clspmv::device_release(p, idle_on);
     }
 };
 
@@ -1553,7 +1554,7 @@ int clspmv_device_coo2bdia_f32(const clspmv_coo_f32* src, clspmv_bdia_f32* dst, 
         return rc;
     if ((rc = cuda_status(cudaMemcpy(bp, bptr.data(), sizeof(int) * bptr.size(), cudaMemcpyHostToDevice)))) return rc;
     O.keep = true;
-    clspmv::device_release(dia.dia_offsets, true);   // the DIA data array becomes the BDIA one
+    clspmv::device_release(dia.dia_offsets, clspmv::kIdleAll);   // the DIA data array becomes the BDIA one
     dst->matinfo = dia.matinfo;
     dst->bdia_band_num = (int)first.size();
     dst->bdia_length = dia.dia_length;

@@ -20,18 +20,19 @@ int upload_array(T** dst, const T* src, size_t n)
     if (clspmv::device_alloc(&p, n * sizeof(T))) return CLSPMV_ERR_ALLOC;
     int rc = cuda_status(cudaMemcpy(p, src, n * sizeof(T), cudaMemcpyHostToDevice));
     if (rc) {
-        clspmv::device_release(p, false);
+        clspmv::device_release(p, clspmv::kIdleNone);
         return rc;
     }
     *dst = static_cast<T*>(p);
     return CLSPMV_OK;
 }
 
-template <class T>
-void release(T*& p)
+// The arrays of one struct, with one wait for the device.
+template <class... T>
+void release(T*&... p)
 {
-    clspmv::device_release(p, false);
-    p = nullptr;
+    int idle_on = clspmv::kIdleNone;
+    ((idle_on = clspmv::device_release(p, idle_on), p = nullptr), ...);
 }
 
 // Uploads the listed arrays in order; on failure frees what was uploaded.
@@ -50,7 +51,7 @@ struct Uploader {
     {
         if (rc)
             for (int i = 0; i < n; i++)
-                clspmv::device_release(done[i], false);
+                clspmv::device_release(done[i], clspmv::kIdleNone);
         return rc;
     }
 };
@@ -186,16 +187,16 @@ int clspmv_upload_sbell_f32(const clspmv_sbell_f32* h, clspmv_sbell_f32* d)
     return u.finish();
 }
 
-int clspmv_device_free_coo_f32(clspmv_coo_f32* d) { if (!d) return CLSPMV_ERR_ARG; release(d->coo_row_id); release(d->coo_col_id); release(d->coo_data); return CLSPMV_OK; }
-int clspmv_device_free_csr_f32(clspmv_csr_f32* d) { if (!d) return CLSPMV_ERR_ARG; release(d->csr_row_ptr); release(d->csr_col_id); release(d->csr_data); return CLSPMV_OK; }
-int clspmv_device_free_dia_f32(clspmv_dia_f32* d) { if (!d) return CLSPMV_ERR_ARG; release(d->dia_offsets); release(d->dia_data); return CLSPMV_OK; }
-int clspmv_device_free_bdia_f32(clspmv_bdia_f32* d) { if (!d) return CLSPMV_ERR_ARG; release(d->bdia_offsets); release(d->bdia_bptr); release(d->bdia_data); return CLSPMV_OK; }
-int clspmv_device_free_ell_f32(clspmv_ell_f32* d) { if (!d) return CLSPMV_ERR_ARG; release(d->ell_col_id); release(d->ell_data); return CLSPMV_OK; }
-int clspmv_device_free_sell_f32(clspmv_sell_f32* d) { if (!d) return CLSPMV_ERR_ARG; release(d->sell_slice_ptr); release(d->sell_col_id); release(d->sell_data); return CLSPMV_OK; }
-int clspmv_device_free_b4csr_f32(clspmv_b4csr_f32* d) { if (!d) return CLSPMV_ERR_ARG; release(d->b4csr_row_ptr); release(d->b4csr_col_id); release(d->b4csr_data); return CLSPMV_OK; }
-int clspmv_device_free_bcsr_f32(clspmv_bcsr_f32* d) { if (!d) return CLSPMV_ERR_ARG; release(d->bcsr_row_ptr); release(d->bcsr_col_id); release(d->bcsr_data); return CLSPMV_OK; }
-int clspmv_device_free_bell_f32(clspmv_bell_f32* d) { if (!d) return CLSPMV_ERR_ARG; release(d->bell_col_id); release(d->bell_data); return CLSPMV_OK; }
-int clspmv_device_free_b4ell_f32(clspmv_b4ell_f32* d) { if (!d) return CLSPMV_ERR_ARG; release(d->b4ell_col_id); release(d->b4ell_data); return CLSPMV_OK; }
-int clspmv_device_free_sbell_f32(clspmv_sbell_f32* d) { if (!d) return CLSPMV_ERR_ARG; release(d->sbell_slice_ptr); release(d->sbell_col_id); release(d->sbell_data); return CLSPMV_OK; }
+int clspmv_device_free_coo_f32(clspmv_coo_f32* d) { if (!d) return CLSPMV_ERR_ARG; release(d->coo_row_id, d->coo_col_id, d->coo_data); return CLSPMV_OK; }
+int clspmv_device_free_csr_f32(clspmv_csr_f32* d) { if (!d) return CLSPMV_ERR_ARG; release(d->csr_row_ptr, d->csr_col_id, d->csr_data); return CLSPMV_OK; }
+int clspmv_device_free_dia_f32(clspmv_dia_f32* d) { if (!d) return CLSPMV_ERR_ARG; release(d->dia_offsets, d->dia_data); return CLSPMV_OK; }
+int clspmv_device_free_bdia_f32(clspmv_bdia_f32* d) { if (!d) return CLSPMV_ERR_ARG; release(d->bdia_offsets, d->bdia_bptr, d->bdia_data); return CLSPMV_OK; }
+int clspmv_device_free_ell_f32(clspmv_ell_f32* d) { if (!d) return CLSPMV_ERR_ARG; release(d->ell_col_id, d->ell_data); return CLSPMV_OK; }
+int clspmv_device_free_sell_f32(clspmv_sell_f32* d) { if (!d) return CLSPMV_ERR_ARG; release(d->sell_slice_ptr, d->sell_col_id, d->sell_data); return CLSPMV_OK; }
+int clspmv_device_free_b4csr_f32(clspmv_b4csr_f32* d) { if (!d) return CLSPMV_ERR_ARG; release(d->b4csr_row_ptr, d->b4csr_col_id, d->b4csr_data); return CLSPMV_OK; }
+int clspmv_device_free_bcsr_f32(clspmv_bcsr_f32* d) { if (!d) return CLSPMV_ERR_ARG; release(d->bcsr_row_ptr, d->bcsr_col_id, d->bcsr_data); return CLSPMV_OK; }
+int clspmv_device_free_bell_f32(clspmv_bell_f32* d) { if (!d) return CLSPMV_ERR_ARG; release(d->bell_col_id, d->bell_data); return CLSPMV_OK; }
+int clspmv_device_free_b4ell_f32(clspmv_b4ell_f32* d) { if (!d) return CLSPMV_ERR_ARG; release(d->b4ell_col_id, d->b4ell_data); return CLSPMV_OK; }
+int clspmv_device_free_sbell_f32(clspmv_sbell_f32* d) { if (!d) return CLSPMV_ERR_ARG; release(d->sbell_slice_ptr, d->sbell_col_id, d->sbell_data); return CLSPMV_OK; }
 
 }  // extern "C"

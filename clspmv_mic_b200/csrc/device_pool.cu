@@ -10,8 +10,8 @@
 // SELL-32 of the power-law matrix of 700k rows in 0.41 instead of 4.0 ms.
 //
 // A kept array has no work pending on it: device_release waits for the
-// device first (as cudaFree does), so it may be used on any stream by any
-// thread. The list holds at most 1/64 of a device's memory (2.9 GB of
+// device first, by what cudaFree waits with (wait_as_free_does), so it may be
+// used on any stream by any thread. The list holds at most 1/64 of a device's memory (2.9 GB of
 // 183 GB) in kKeptMost arrays, the oldest leaving first; it is given back
 // when an allocation fails, when less than 1/8 of the device is left after
 // a large new one, and by clspmv_device_trim. Only arrays that device_alloc made
@@ -45,6 +45,7 @@ std::mutex g_mu;
 std::list<Kept> g_kept;                              // oldest first
 std::unordered_map<int, size_t> g_kept_bytes;        // per device
 std::unordered_map<void*, Made> g_made;              // arrays made by device_alloc and not yet cudaFree'd
+std::unordered_map<int, Kept> g_marker;              // wait_as_free_does, per device
 
 constexpr size_t kGrain = 512;
 constexpr size_t kLarge = 64u << 20;
@@ -114,6 +115,14 @@ std::list<Kept> take_kept(int device)
         out.push_back(*it);
         it = unlist(it, false);
     }
+    for (auto it = g_marker.begin(); it != g_marker.end();) {
+        if (device >= 0 && it->first != device) {
+            ++it;
+            continue;
+        }
+        out.push_back(it->second);
+        it = g_marker.erase(it);
+    }
     return out;
 }
 
@@ -121,6 +130,27 @@ void free_all(const std::list<Kept>& l)
 {
     for (const Kept& k : l)
         if (alive(k) && cudaFree(k.p) != cudaSuccess) cudaGetLastError();
+}
+
+// Waits for all work of the current device by freeing a small allocation:
+// cudaFree waits for it, and is allowed where another thread captures a
+// stream in its own (thread-local) mode, or any thread in relaxed mode.
+// cudaDeviceSynchronize, the cheaper wait (1.8 against 4 us on B200), fails
+// there and spoils the capture. Another small allocation is made first, so
+// that their page of the device stays mapped.
+bool wait_as_free_does(int device)
+{
+    Kept last, next{nullptr, kGrain, device, 0};
+    if (cudaMalloc(&next.p, kGrain) != cudaSuccess) return false;
+    next.id = allocation_id(next.p);
+    {
+        std::lock_guard<std::mutex> lock(g_mu);
+        auto at = g_marker.emplace(device, Kept{nullptr, kGrain, device, 0}).first;
+        last = at->second;
+        at->second = next;
+    }
+    if ((!last.p || !alive(last)) && cudaMalloc(&last.p, kGrain) != cudaSuccess) return false;
+    return cudaFree(last.p) == cudaSuccess;
 }
 
 }  // namespace
@@ -166,15 +196,15 @@ int device_alloc(void** out, size_t bytes)
     return CLSPMV_OK;
 }
 
-void device_release(void* p, bool idle)
+int device_release(void* p, int idle_on)
 {
-    if (!p) return;
+    if (!p) return idle_on;
     Made made{0, 0};
     const unsigned long long id = allocation_id(p);
     {
         std::lock_guard<std::mutex> lock(g_mu);
         for (const Kept& k : g_kept)
-            if (k.p == p && k.id == id) return;   // released already
+            if (k.p == p && k.id == id) return idle_on;   // released already
         auto it = g_made.find(p);
         if (it != g_made.end() && it->second.id == id) made = it->second;
     }
@@ -184,11 +214,12 @@ void device_release(void* p, bool idle)
     const size_t limit = keep ? limit_of(at.device) : 0;
     if (keep) keep = bytes <= limit;
     int cur = -1;
-    if (keep) {
+    if (keep && idle_on != kIdleAll && idle_on != at.device) {
         cudaGetDevice(&cur);
         if (cur != at.device) cudaSetDevice(at.device);
-        if (!idle) keep = cudaDeviceSynchronize() == cudaSuccess;
+        keep = wait_as_free_does(at.device);
         if (cur >= 0 && cur != at.device) cudaSetDevice(cur);
+        if (keep) idle_on = at.device;
     }
     if (!keep) {
         cudaGetLastError();
@@ -197,7 +228,7 @@ void device_release(void* p, bool idle)
             g_made.erase(p);
         }
         if (cudaFree(p) != cudaSuccess) cudaGetLastError();
-        return;
+        return idle_on;
     }
     std::list<Kept> drop;
     {
@@ -207,7 +238,7 @@ void device_release(void* p, bool idle)
                 ++it;
                 continue;
             }
-            if (it->id == id) return;
+            if (it->id == id) return idle_on;
             it = unlist(it, false);   // an array that is gone, whose address this one has
         }
         g_kept.push_back(Kept{p, bytes, at.device, id});
@@ -223,6 +254,7 @@ void device_release(void* p, bool idle)
         }
     }
     free_all(drop);
+    return idle_on;
 }
 
 }  // namespace clspmv

@@ -129,13 +129,13 @@ static constexpr size_t MB = 1 << 20;
 static void reuse()   // kept for the next request that it fits, given back by trim
 {
     void* a = make(MB);
-    device_release(a, true);
+    device_release(a, clspmv::kIdleAll);
     CHECK(fake::live(a) && make(MB) == a);
-    device_release(a, true);
-    device_release(a, true);   // a second release of the same array
+    device_release(a, clspmv::kIdleAll);
+    device_release(a, clspmv::kIdleAll);   // a second release of the same array
     void *b = make(MB), *c = make(MB);
     CHECK(b != c);
-    device_release(b, true);
+    device_release(b, clspmv::kIdleAll);
     CHECK(make(2 * MB) != b);
     clspmv_device_trim();
     CHECK(!fake::live(b) && fake::live(c));
@@ -145,32 +145,32 @@ static void bounds()   // 1/64 of the device and 256 arrays, the oldest leave fi
 {
     std::vector<void*> p;
     for (int i = 0; i < 12; i++) p.push_back(make(100 * MB));
-    for (void* q : p) device_release(q, true);
+    for (void* q : p) device_release(q, clspmv::kIdleAll);
     size_t held = 0;
     for (void* q : p) held += fake::live(q) ? 100 * MB : 0;
     CHECK(held <= fake::total / 64 && held + 100 * MB > fake::total / 64 && !fake::live(p[0]) && fake::live(p[11]));
     clspmv_device_trim();
     p.clear();
     for (int i = 0; i < 300; i++) p.push_back(make(4096));
-    for (void* q : p) device_release(q, true);
+    for (void* q : p) device_release(q, clspmv::kIdleAll);
     int n = 0;
     for (void* q : p) n += fake::live(q);
     CHECK(n <= 256 && n >= 250 && fake::live(p[299]));
     clspmv_device_trim();
     void* big = make(fake::total / 32);   // more than the list may hold
-    device_release(big, true);
+    device_release(big, clspmv::kIdleAll);
     CHECK(!fake::live(big));
 }
 
 static void low_memory()   // given back for an allocation that fails, and when little is left after a large one
 {
     void* a = make(500 * MB);
-    device_release(a, true);
+    device_release(a, clspmv::kIdleAll);
     void* rest = nullptr;
     CHECK(device_alloc(&rest, fake::total - 200 * MB) == CLSPMV_OK && !fake::live(a));
     cudaFree(rest);
     a = make(500 * MB);
-    device_release(a, true);
+    device_release(a, clspmv::kIdleAll);
     rest = make(fake::total - fake::total / 8);
     CHECK(!fake::live(a));
 }
@@ -178,14 +178,14 @@ static void low_memory()   // given back for an allocation that fails, and when 
 static void reset()   // kept arrays that a device reset took away
 {
     void *a = make(MB), *b = make(3 * MB);
-    device_release(a, true);
-    device_release(b, true);
+    device_release(a, clspmv::kIdleAll);
+    device_release(b, clspmv::kIdleAll);
     fake::vanish();
     void* mine = nullptr;
     CHECK(cudaMalloc(&mine, MB) == cudaSuccess && mine == a);   // the address belongs to the caller now
     void *c = make(MB), *d = make(3 * MB);
     CHECK(c != mine && fake::live(d));
-    device_release(c, true);
+    device_release(c, clspmv::kIdleAll);
     CHECK(make(MB) == c);
     clspmv_device_trim();
     CHECK(fake::live(mine) && fake::live(c) && fake::live(d) && fake::bad_frees == 0);
@@ -197,15 +197,47 @@ static void freed_by_the_caller()   // an array the caller freed, whose address 
     cudaFree(a);
     void* mine = nullptr;
     CHECK(cudaMalloc(&mine, MB) == cudaSuccess && mine == a);
-    device_release(mine, true);   // no array of device_alloc: freed
+    device_release(mine, clspmv::kIdleAll);   // no array of device_alloc: freed
     CHECK(!fake::live(mine));
     a = make(MB);
-    device_release(a, true);
+    device_release(a, clspmv::kIdleAll);
     cudaFree(a);
     CHECK(cudaMalloc(&mine, MB) == cudaSuccess && mine == a);
     CHECK(make(MB) != mine);
     clspmv_device_trim();
     CHECK(fake::live(mine));
+}
+
+static void waits()   // nothing is kept with work in flight; one wait for arrays released together
+{
+    void *a = make(MB), *b = make(MB);
+    fake::working = true;
+    const int idle_on = device_release(a, clspmv::kIdleNone);
+    CHECK(!fake::working && fake::live(a) && idle_on == 0);
+    fake::working = true;
+    CHECK(device_release(b, idle_on) == 0 && fake::working && fake::live(b));
+    void* c = make(MB);
+    fake::vanish();   // and with it what the wait keeps
+    void* mine = nullptr;
+    CHECK(cudaMalloc(&mine, 512) == cudaSuccess);
+    c = make(MB);
+    fake::working = true;
+    device_release(c, clspmv::kIdleNone);
+    CHECK(!fake::working && fake::live(mine) && fake::bad_frees == 0);
+    clspmv_device_trim();
+    CHECK(fake::blocks().size() == 1 && fake::live(mine));
+}
+
+static void capture()   // a release while another thread captures a stream
+{
+    void *a = make(MB), *b = make(MB);
+    fake::working = fake::capturing = true;
+    device_release(a, clspmv::kIdleNone);
+    CHECK(!fake::invalidated && !fake::working);
+    fake::working = fake::forbidden = true;   // as cudaFree: refused, and not handed out
+    device_release(b, clspmv::kIdleNone);
+    fake::capturing = fake::forbidden = false;
+    CHECK(make(MB) == a && make(MB) != b);
 }
 
 int main(int argc, char** argv)
@@ -216,6 +248,8 @@ int main(int argc, char** argv)
     else if (what == "low_memory") low_memory();
     else if (what == "reset") reset();
     else if (what == "freed_by_the_caller") freed_by_the_caller();
+    else if (what == "waits") waits();
+    else if (what == "capture") capture();
     else return 99;
     return failures;
 }

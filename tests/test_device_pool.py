@@ -1,7 +1,8 @@
 """The list of kept device arrays (csrc/device_pool.cu), compiled against a
 stand-in for the CUDA calls it makes (compat/device_pool_check.cpp): no GPU.
 An array that a device reset took away or that the caller freed is not handed
-out and not freed again; the list's bounds and who leaves it hold."""
+out and not freed again; the list's bounds and who leaves it hold; a release
+waits for the device without spoiling another thread's stream capture."""
 import subprocess
 
 import pytest
@@ -22,6 +23,6 @@ def check(tmp_path_factory):
     return run
 
 
-@pytest.mark.parametrize("name", ["reuse", "bounds", "low_memory", "reset", "freed_by_the_caller"])
+@pytest.mark.parametrize("name", ["reuse", "bounds", "low_memory", "reset", "freed_by_the_caller", "waits", "capture"])
 def test_kept_arrays(check, name):
     check(name)
