@@ -41,11 +41,13 @@ struct Made {
     unsigned long long id;
 };
 
-std::mutex g_mu;
-std::list<Kept> g_kept;                              // oldest first
-std::unordered_map<int, size_t> g_kept_bytes;        // per device
-std::unordered_map<void*, Made> g_made;              // arrays made by device_alloc and not yet cudaFree'd
-std::unordered_map<int, Kept> g_marker;              // wait_as_free_does, per device
+// Never destroyed: a matrix may be released by a destructor that runs after this file's would have.
+std::mutex& g_mu = *new std::mutex;
+std::list<Kept>& g_kept = *new std::list<Kept>;      // oldest first
+std::list<Kept>& g_marker = *new std::list<Kept>;    // wait_as_free_does, one per device
+auto& g_kept_bytes = *new std::unordered_map<int, size_t>;   // per device
+auto& g_made = *new std::unordered_map<void*, Made>;         // arrays made by device_alloc and not yet cudaFree'd
+auto& g_limit = *new std::unordered_map<int, size_t>;        // limit_of, per device
 
 constexpr size_t kGrain = 512;
 constexpr size_t kLarge = 64u << 20;
@@ -53,11 +55,9 @@ constexpr size_t kKeptMost = 256;   // arrays on the list, so that a search stay
 
 size_t limit_of(int device)
 {
-    static std::mutex mu;
-    static std::unordered_map<int, size_t> cache;
-    std::lock_guard<std::mutex> lock(mu);
-    auto it = cache.find(device);
-    if (it != cache.end()) return it->second;
+    std::lock_guard<std::mutex> lock(g_mu);
+    auto it = g_limit.find(device);
+    if (it != g_limit.end()) return it->second;
     size_t fr = 0, total = 0;
     int cur = -1;
     cudaGetDevice(&cur);
@@ -67,7 +67,7 @@ size_t limit_of(int device)
         total = 0;
     }
     if (cur >= 0 && cur != device) cudaSetDevice(cur);
-    return cache[device] = total / 64;
+    return g_limit[device] = total / 64;
 }
 
 // The driver's id of the allocation at p, 0 if there is none (0.14 us).
@@ -91,15 +91,21 @@ unsigned long long allocation_id(void* p)
 
 bool alive(const Kept& k) { return allocation_id(k.p) == k.id; }
 
-// Takes an entry off the list (g_mu held), and off the arrays made unless it is handed out.
-std::list<Kept>::iterator unlist(std::list<Kept>::iterator it, bool handed_out)
+// Moves an entry from the list to `out` (g_mu held); returns the next one. Allocates nothing.
+std::list<Kept>::iterator unlist(std::list<Kept>::iterator it, std::list<Kept>& out)
 {
-    g_kept_bytes[it->device] -= it->bytes;
-    if (!handed_out) {
-        auto made = g_made.find(it->p);
-        if (made != g_made.end() && made->second.id == it->id) g_made.erase(made);
-    }
-    return g_kept.erase(it);
+    auto held = g_kept_bytes.find(it->device);
+    if (held != g_kept_bytes.end()) held->second -= it->bytes;
+    auto next = std::next(it);
+    out.splice(out.end(), g_kept, it);
+    return next;
+}
+// ... and off the arrays made.
+std::list<Kept>::iterator forget(std::list<Kept>::iterator it, std::list<Kept>& out)
+{
+    auto made = g_made.find(it->p);
+    if (made != g_made.end() && made->second.id == it->id) g_made.erase(made);
+    return unlist(it, out);
 }
 
 // Takes the kept arrays of `device` (all devices: -1) off the list.
@@ -107,21 +113,12 @@ std::list<Kept> take_kept(int device)
 {
     std::list<Kept> out;
     std::lock_guard<std::mutex> lock(g_mu);
-    for (auto it = g_kept.begin(); it != g_kept.end();) {
-        if (device >= 0 && it->device != device) {
-            ++it;
-            continue;
-        }
-        out.push_back(*it);
-        it = unlist(it, false);
-    }
+    for (auto it = g_kept.begin(); it != g_kept.end();)
+        it = device < 0 || it->device == device ? forget(it, out) : std::next(it);
     for (auto it = g_marker.begin(); it != g_marker.end();) {
-        if (device >= 0 && it->first != device) {
-            ++it;
-            continue;
-        }
-        out.push_back(it->second);
-        it = g_marker.erase(it);
+        auto next = std::next(it);
+        if (device < 0 || it->device == device) out.splice(out.end(), g_marker, it);
+        it = next;
     }
     return out;
 }
@@ -129,7 +126,7 @@ std::list<Kept> take_kept(int device)
 void free_all(const std::list<Kept>& l)
 {
     for (const Kept& k : l)
-        if (alive(k) && cudaFree(k.p) != cudaSuccess) cudaGetLastError();
+        if (k.p && alive(k) && cudaFree(k.p) != cudaSuccess) cudaGetLastError();
 }
 
 // Waits for all work of the current device by freeing a small allocation:
@@ -140,17 +137,69 @@ void free_all(const std::list<Kept>& l)
 // that their page of the device stays mapped.
 bool wait_as_free_does(int device)
 {
+    auto marker_of = [&]() -> Kept& {   // g_mu held
+        for (Kept& k : g_marker)
+            if (k.device == device) return k;
+        g_marker.push_back(Kept{nullptr, kGrain, device, 0});
+        return g_marker.back();
+    };
+    {
+        std::lock_guard<std::mutex> lock(g_mu);
+        marker_of();
+    }
     Kept last, next{nullptr, kGrain, device, 0};
     if (cudaMalloc(&next.p, kGrain) != cudaSuccess) return false;
     next.id = allocation_id(next.p);
     {
         std::lock_guard<std::mutex> lock(g_mu);
-        auto at = g_marker.emplace(device, Kept{nullptr, kGrain, device, 0}).first;
-        last = at->second;
-        at->second = next;
+        Kept& m = marker_of();
+        last = m;
+        m = next;
     }
     if ((!last.p || !alive(last)) && cudaMalloc(&last.p, kGrain) != cudaSuccess) return false;
     return cudaFree(last.p) == cudaSuccess;
+}
+
+// Puts an array on the list; false where it has to be freed instead.
+bool keep_array(void* p, int* idle_on)
+{
+    const unsigned long long id = allocation_id(p);
+    size_t bytes = 0;
+    {
+        std::lock_guard<std::mutex> lock(g_mu);
+        for (const Kept& k : g_kept)
+            if (k.p == p && k.id == id) return true;   // released already
+        auto it = g_made.find(p);
+        if (id && it != g_made.end() && it->second.id == id) bytes = it->second.bytes;
+    }
+    cudaPointerAttributes at{};
+    if (!bytes || cudaPointerGetAttributes(&at, p) != cudaSuccess || at.type != cudaMemoryTypeDevice) return false;
+    const size_t limit = limit_of(at.device);
+    if (bytes > limit) return false;
+    if (*idle_on != kIdleAll && *idle_on != at.device) {
+        int cur = -1;
+        cudaGetDevice(&cur);
+        if (cur != at.device) cudaSetDevice(at.device);
+        const bool idle = wait_as_free_does(at.device);
+        if (cur >= 0 && cur != at.device) cudaSetDevice(cur);
+        if (!idle) return false;
+        *idle_on = at.device;
+    }
+    std::list<Kept> drop, gone;
+    {
+        std::lock_guard<std::mutex> lock(g_mu);
+        for (auto it = g_kept.begin(); it != g_kept.end();) {
+            if (it->p == p && it->id == id) return true;
+            it = it->p == p ? forget(it, gone) : std::next(it);   // gone: its address is this one's
+        }
+        size_t& held = g_kept_bytes[at.device];
+        g_kept.push_back(Kept{p, bytes, at.device, id});
+        held += bytes;
+        for (auto it = g_kept.begin(); (held > limit || g_kept.size() > kKeptMost) && it != g_kept.end();)
+            it = it->device == at.device ? forget(it, drop) : std::next(it);
+    }
+    free_all(drop);
+    return true;
 }
 
 }  // namespace
@@ -163,6 +212,7 @@ int device_alloc(void** out, size_t bytes)
     cudaGetDevice(&device);
     {
         // the smallest kept array that holds the request and is at most 1/8 larger
+        std::list<Kept> gone;
         std::lock_guard<std::mutex> lock(g_mu);
         const size_t most = bytes + bytes / 8 + kGrain;
         while (true) {
@@ -171,10 +221,12 @@ int device_alloc(void** out, size_t bytes)
                 if (it->device == device && it->bytes >= bytes && it->bytes <= most && (best == g_kept.end() || it->bytes < best->bytes))
                     best = it;
             if (best == g_kept.end()) break;
-            const bool ok = alive(*best);
-            if (ok) *out = best->p;
-            unlist(best, ok);
-            if (ok) return CLSPMV_OK;
+            if (alive(*best)) {
+                *out = best->p;
+                unlist(best, gone);
+                return CLSPMV_OK;
+            }
+            forget(best, gone);
         }
     }
     void* p = nullptr;
@@ -186,9 +238,13 @@ int device_alloc(void** out, size_t bytes)
             return CLSPMV_ERR_ALLOC;
         }
     }
-    {
+    try {
+        const Made made{bytes, allocation_id(p)};
         std::lock_guard<std::mutex> lock(g_mu);
-        g_made[p] = Made{bytes, allocation_id(p)};
+        g_made[p] = made;
+    } catch (...) {   // the host is out of memory
+        if (cudaFree(p) != cudaSuccess) cudaGetLastError();
+        return CLSPMV_ERR_ALLOC;
     }
     size_t fr = 0, total = 0;
     if (bytes >= kLarge && cudaMemGetInfo(&fr, &total) == cudaSuccess && fr < total / 8) free_all(take_kept(device));
@@ -199,61 +255,16 @@ int device_alloc(void** out, size_t bytes)
 int device_release(void* p, int idle_on)
 {
     if (!p) return idle_on;
-    Made made{0, 0};
-    const unsigned long long id = allocation_id(p);
+    try {
+        if (keep_array(p, &idle_on)) return idle_on;
+    } catch (...) {   // the host is out of memory
+    }
+    cudaGetLastError();
     {
         std::lock_guard<std::mutex> lock(g_mu);
-        for (const Kept& k : g_kept)
-            if (k.p == p && k.id == id) return idle_on;   // released already
-        auto it = g_made.find(p);
-        if (it != g_made.end() && it->second.id == id) made = it->second;
+        g_made.erase(p);
     }
-    const size_t bytes = made.bytes;
-    cudaPointerAttributes at{};
-    bool keep = id && bytes && cudaPointerGetAttributes(&at, p) == cudaSuccess && at.type == cudaMemoryTypeDevice;
-    const size_t limit = keep ? limit_of(at.device) : 0;
-    if (keep) keep = bytes <= limit;
-    int cur = -1;
-    if (keep && idle_on != kIdleAll && idle_on != at.device) {
-        cudaGetDevice(&cur);
-        if (cur != at.device) cudaSetDevice(at.device);
-        keep = wait_as_free_does(at.device);
-        if (cur >= 0 && cur != at.device) cudaSetDevice(cur);
-        if (keep) idle_on = at.device;
-    }
-    if (!keep) {
-        cudaGetLastError();
-        {
-            std::lock_guard<std::mutex> lock(g_mu);
-            g_made.erase(p);
-        }
-        if (cudaFree(p) != cudaSuccess) cudaGetLastError();
-        return idle_on;
-    }
-    std::list<Kept> drop;
-    {
-        std::lock_guard<std::mutex> lock(g_mu);
-        for (auto it = g_kept.begin(); it != g_kept.end();) {
-            if (it->p != p) {
-                ++it;
-                continue;
-            }
-            if (it->id == id) return idle_on;
-            it = unlist(it, false);   // an array that is gone, whose address this one has
-        }
-        g_kept.push_back(Kept{p, bytes, at.device, id});
-        size_t& held = g_kept_bytes[at.device];
-        held += bytes;
-        for (auto it = g_kept.begin(); (held > limit || g_kept.size() > kKeptMost) && it != g_kept.end();) {
-            if (it->device != at.device) {
-                ++it;
-                continue;
-            }
-            drop.push_back(*it);
-            it = unlist(it, false);
-        }
-    }
-    free_all(drop);
+    if (cudaFree(p) != cudaSuccess) cudaGetLastError();
     return idle_on;
 }
 

@@ -13,6 +13,21 @@
 #include <string>
 #include <vector>
 
+static int fail_new = -1;   // allocations of the host until one fails, -1: none does
+void* operator new(size_t n)
+{
+    if (fail_new >= 0 && fail_new-- == 0) throw std::bad_alloc();
+    if (void* p = malloc(n ? n : 1)) return p;
+    throw std::bad_alloc();
+}
+void operator delete(void* p) noexcept { free(p); }
+void operator delete(void* p, size_t) noexcept { free(p); }
+struct Unfailing {   // the stand-in's own allocations
+    int was = fail_new;
+    Unfailing() { fail_new = -1; }
+    ~Unfailing() { fail_new = was; }
+};
+
 namespace fake {
 struct Block {
     size_t bytes;
@@ -46,6 +61,7 @@ cudaError_t CUDARTAPI cudaGetLastError(void) { return cudaSuccess; }
 cudaError_t CUDARTAPI cudaMemGetInfo(size_t* f, size_t* t) { *f = fake::total - fake::used; *t = fake::total; return cudaSuccess; }
 cudaError_t CUDARTAPI cudaMalloc(void** p, size_t n)
 {
+    Unfailing u;
     if (fake::forbidden) { fake::invalidated = true; return cudaErrorStreamCaptureUnsupported; }
     if (fake::used + n > fake::total) return cudaErrorMemoryAllocation;
     auto hole = fake::holes().find(n);
@@ -63,6 +79,7 @@ cudaError_t CUDARTAPI cudaMalloc(void** p, size_t n)
 }
 cudaError_t CUDARTAPI cudaFree(void* p)
 {
+    Unfailing u;
     if (fake::forbidden) { fake::invalidated = true; return cudaErrorStreamCaptureUnsupported; }
     if (!p) return cudaSuccess;
     auto it = fake::blocks().find(static_cast<char*>(p));
@@ -108,6 +125,17 @@ cudaError_t CUDARTAPI cudaGetDriverEntryPoint(const char* name, void** fn, unsig
     return cudaSuccess;
 }
 }
+
+namespace clspmv { int device_release(void* p, int idle_on); }
+static struct AtExit {   // made before, so destroyed after, whatever the included file makes
+    void* array = nullptr;
+    ~AtExit()
+    {
+        if (!array) return;
+        clspmv::device_release(array, -1);
+        if (!fake::live(array)) _Exit(1);   // kept, as at any other time
+    }
+} at_exit;
 
 #include "device_pool.cu"
 
@@ -240,6 +268,32 @@ static void capture()   // a release while another thread captures a stream
     CHECK(make(MB) == a && make(MB) != b);
 }
 
+static void host_memory()   // no exception leaves a call, and no array is lost
+{
+    for (int n = 0; n < 12; n++) {
+        void *a = nullptr, *b = make(3 * MB), *c = nullptr;
+        bool threw = false;
+        fail_new = n;
+        try {
+            device_alloc(&a, MB);
+            device_release(b, clspmv::kIdleNone);
+            device_release(a, clspmv::kIdleNone);
+            device_alloc(&c, 2 * MB);
+            device_release(c, clspmv::kIdleAll);
+            clspmv_device_trim();
+        } catch (...) {
+            threw = true;
+        }
+        fail_new = -1;
+        CHECK(!threw);
+        clspmv_device_trim();
+        CHECK(fake::blocks().empty());
+        fake::vanish();
+    }
+}
+
+static void at_exit_check() { at_exit.array = make(MB); }
+
 int main(int argc, char** argv)
 {
     const std::string what = argc > 1 ? argv[1] : "";
@@ -250,6 +304,8 @@ int main(int argc, char** argv)
     else if (what == "freed_by_the_caller") freed_by_the_caller();
     else if (what == "waits") waits();
     else if (what == "capture") capture();
+    else if (what == "host_memory") host_memory();
+    else if (what == "at_exit") at_exit_check();
     else return 99;
     return failures;
 }

@@ -2,7 +2,9 @@
 stand-in for the CUDA calls it makes (compat/device_pool_check.cpp): no GPU.
 An array that a device reset took away or that the caller freed is not handed
 out and not freed again; the list's bounds and who leaves it hold; a release
-waits for the device without spoiling another thread's stream capture."""
+waits for the device without spoiling another thread's stream capture; no
+exception leaves a call when the host is out of memory; a matrix may be
+released after the library's own destructors."""
 import subprocess
 
 import pytest
@@ -23,6 +25,6 @@ def check(tmp_path_factory):
     return run
 
 
-@pytest.mark.parametrize("name", ["reuse", "bounds", "low_memory", "reset", "freed_by_the_caller", "waits", "capture"])
+@pytest.mark.parametrize("name", ["reuse", "bounds", "low_memory", "reset", "freed_by_the_caller", "waits", "capture", "host_memory", "at_exit"])
 def test_kept_arrays(check, name):
     check(name)
