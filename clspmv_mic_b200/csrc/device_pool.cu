@@ -11,14 +11,17 @@
 //
 // A kept array has no work pending on it: device_release waits for the
 // device first, by what cudaFree waits with (wait_as_free_does), so it may be
-// used on any stream by any thread. The list holds at most 1/64 of a device's memory (2.9 GB of
-// 183 GB) in kKeptMost arrays, the oldest leaving first; it is given back
-// when an allocation fails, when less than 1/8 of the device is left after
-// a large new one, and by clspmv_device_trim. Only arrays that device_alloc made
-// are kept; any other pointer goes to cudaFree. An array is known by the
-// driver's id of its allocation, which no other one of the process gets: one
-// that the caller freed, or that a device reset took away, is neither handed
-// out nor freed again, whoever owns its address by then.
+// used on any stream by any thread. The list holds at most 1/64 of a device's
+// memory (2.9 GB of 183 GB) in kKeptMost arrays, the oldest leaving first. It
+// is given back when an allocation fails, when less than 1/8 of the device is
+// left after a large new one or once the list has grown by kLarge since the
+// last look (asking the driver takes 0.1 to 0.3 ms), and by clspmv_device_trim.
+//
+// Only arrays that device_alloc made are kept; any other pointer goes to
+// cudaFree. An array is known by the driver's id of its allocation, which no
+// other one of the process gets: one that the caller freed, or that a device
+// reset took away, is neither handed out nor freed again, whoever owns its
+// address by then.
 #include <cuda.h>
 #include <algorithm>
 #include <list>
@@ -47,6 +50,7 @@ std::list<Kept>& g_kept = *new std::list<Kept>;      // oldest first
 std::list<Kept>& g_marker = *new std::list<Kept>;    // wait_as_free_does, one per device
 auto& g_kept_bytes = *new std::unordered_map<int, size_t>;   // per device
 auto& g_made = *new std::unordered_map<void*, Made>;         // arrays made by device_alloc and not yet cudaFree'd
+auto& g_seen = *new std::unordered_map<int, size_t>;         // bytes kept when the device's free memory was last looked at
 auto& g_limit = *new std::unordered_map<int, size_t>;        // limit_of, per device
 
 constexpr size_t kGrain = 512;
@@ -120,6 +124,8 @@ std::list<Kept> take_kept(int device)
         if (device < 0 || it->device == device) out.splice(out.end(), g_marker, it);
         it = next;
     }
+    for (auto& seen : g_seen)
+        if (device < 0 || seen.first == device) seen.second = 0;
     return out;
 }
 
@@ -160,6 +166,13 @@ bool wait_as_free_does(int device)
     return cudaFree(last.p) == cudaSuccess;
 }
 
+// Gives the kept arrays of the current device back when less than 1/8 of it is left.
+void give_back_if_short(int device)
+{
+    size_t fr = 0, total = 0;
+    if (cudaMemGetInfo(&fr, &total) == cudaSuccess && fr < total / 8) free_all(take_kept(device));
+}
+
 // Puts an array on the list; false where it has to be freed instead.
 bool keep_array(void* p, int* idle_on)
 {
@@ -186,8 +199,10 @@ bool keep_array(void* p, int* idle_on)
         *idle_on = at.device;
     }
     std::list<Kept> drop, gone;
+    bool look = false;
     {
         std::lock_guard<std::mutex> lock(g_mu);
+        size_t& seen = g_seen[at.device];
         for (auto it = g_kept.begin(); it != g_kept.end();) {
             if (it->p == p && it->id == id) return true;
             it = it->p == p ? forget(it, gone) : std::next(it);   // gone: its address is this one's
@@ -197,8 +212,17 @@ bool keep_array(void* p, int* idle_on)
         held += bytes;
         for (auto it = g_kept.begin(); (held > limit || g_kept.size() > kKeptMost) && it != g_kept.end();)
             it = it->device == at.device ? forget(it, drop) : std::next(it);
+        look = held >= seen + kLarge;
+        if (look) seen = held;
     }
     free_all(drop);
+    if (look) {
+        int cur = -1;
+        cudaGetDevice(&cur);
+        if (cur != at.device) cudaSetDevice(at.device);
+        give_back_if_short(at.device);
+        if (cur >= 0 && cur != at.device) cudaSetDevice(cur);
+    }
     return true;
 }
 
@@ -246,8 +270,7 @@ int device_alloc(void** out, size_t bytes)
         if (cudaFree(p) != cudaSuccess) cudaGetLastError();
         return CLSPMV_ERR_ALLOC;
     }
-    size_t fr = 0, total = 0;
-    if (bytes >= kLarge && cudaMemGetInfo(&fr, &total) == cudaSuccess && fr < total / 8) free_all(take_kept(device));
+    if (bytes >= kLarge) give_back_if_short(device);
     *out = p;
     return CLSPMV_OK;
 }

@@ -256,7 +256,8 @@ void clspmv_free_sbell_f32(clspmv_sbell_f32* m);
 /* and releases those arrays; a bounded number of released ones (1/64 of a  */
 /* device's memory) is kept for the next upload or conversion and given     */
 /* back by clspmv_device_trim, when an allocation of this library fails, or */
-/* when under 1/8 of the device is left after a large new one.              */
+/* when under 1/8 of the device is found left, after a large new array or   */
+/* when the kept ones grow. A device reset takes the kept ones with it.     */
 /* Replaces the ALLOCATE_GPU_READ uploads of the per-format drivers         */
 /* (include/oclcommon.h:13-38) and the cpy_<fmt>_mat helpers of             */
 /* src/spmv_cocktail.cpp:304-1009.                                          */

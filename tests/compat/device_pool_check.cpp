@@ -201,6 +201,15 @@ static void low_memory()   // given back for an allocation that fails, and when 
     device_release(a, clspmv::kIdleAll);
     rest = make(fake::total - fake::total / 8);
     CHECK(!fake::live(a));
+    cudaFree(rest);
+    a = make(500 * MB);   // little is left after allocations that are not this library's
+    CHECK(cudaMalloc(&rest, fake::total - fake::total / 8) == cudaSuccess);
+    device_release(a, clspmv::kIdleAll);
+    CHECK(!fake::live(a));
+    cudaFree(rest);
+    a = make(500 * MB);
+    device_release(a, clspmv::kIdleAll);
+    CHECK(fake::live(a));
 }
 
 static void reset()   // kept arrays that a device reset took away
