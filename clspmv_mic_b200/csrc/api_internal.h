@@ -49,16 +49,18 @@ int launch_diag_bulk(int rows, int cols, int ndiag, int len, const int* offsets,
 
 // Steps of y <- alpha*A*x + beta*y; x <- y of a DIA / BDIA matrix of `ndiag` diagonals held by one cluster's shared
 // memory, in one launch (iterate_resident.cu); x holds at least as many entries as y.
-bool resident_iterate_fits(int rows, int ndiag);
-int resident_iterate_dia(const clspmv_dia_f32* m, float* x, float* y, float alpha, float beta, int steps, cudaStream_t st);
-struct ResidentRows {
-    int ctas = 0, per = 0, cap = 0;   // CTAs of the cluster (0: the matrix does not fit), rows and most entries of one
+// The plans are made where the matrix is uploaded, with its device current.
+struct ResidentPlan {
+    int ctas = 0, per = 0, cap = 0;   // CTAs of the cluster (0: the matrix does not fit), rows and most entries of one (COO, CSR)
 };
+ResidentPlan resident_dia_plan(int rows, int ndiag);
 // COO (sorted row ids) or CSR (row pointer), from the host arrays.
-ResidentRows resident_rows_plan(int rows, int nnz, const int* row_id, const int* row_ptr);
-int resident_iterate_coo(const clspmv_coo_f32* m, const ResidentRows& p, float* x, float* y, float alpha, float beta, int steps, cudaStream_t st);
-int resident_iterate_csr(const clspmv_csr_f32* m, const ResidentRows& p, float* x, float* y, float alpha, float beta, int steps, cudaStream_t st);
-int resident_iterate_bdia(const clspmv_bdia_f32* m, int ndiag, float* x, float* y, float alpha, float beta, int steps, cudaStream_t st);
+ResidentPlan resident_rows_plan(int rows, int nnz, const int* row_id, const int* row_ptr);
+int resident_iterate_dia(const clspmv_dia_f32* m, const ResidentPlan& p, float* x, float* y, float alpha, float beta, int steps, cudaStream_t st);
+int resident_iterate_bdia(const clspmv_bdia_f32* m, int ndiag, const ResidentPlan& p, float* x, float* y, float alpha, float beta, int steps,
+                          cudaStream_t st);
+int resident_iterate_coo(const clspmv_coo_f32* m, const ResidentPlan& p, float* x, float* y, float alpha, float beta, int steps, cudaStream_t st);
+int resident_iterate_csr(const clspmv_csr_f32* m, const ResidentPlan& p, float* x, float* y, float alpha, float beta, int steps, cudaStream_t st);
 
 // Fused Cocktail SpMV (cocktail_fused.cu): the parts of a partitioned matrix
 // (device struct) cut into tiles, interleaved into one work list and run by

@@ -27,7 +27,7 @@ struct clspmv_cocktail_handle {
     int* chunk_plan = nullptr;        // first row of every nonzero chunk of the CSR part
     int nparts = 0;
     int bdia_ndiag = 0;               // diagonals of the BDIA part
-    ResidentRows rows;                // how a lone COO / CSR part fits a cluster
+    ResidentPlan resident;            // how a lone DIA, BDIA, COO or CSR part fits a cluster
     FusedPlan* fused = nullptr;       // one persistent launch over all parts (two or more parts)
     clspmv_sell_plan* sell_plan = nullptr;   // the SELL part's length plan, when it reads well under the stored slots
     int schedule = CLSPMV_SCHEDULE_AUTO;
@@ -161,15 +161,11 @@ constexpr int kResidentSteps = 4;
 int resident_steps(clspmv_cocktail_handle* h, float* x, float* y, float alpha, float beta, int steps, cudaStream_t st)
 {
     const clspmv_cocktail_f32& d = h->dev;
-    if (h->nparts != 1 || steps < kResidentSteps) return CLSPMV_ERR_UNSUPPORTED;
-    if (d.ifusedia && d.dia.matinfo.height == d.mat_height && d.mat_height <= d.dia.dia_length_aligned &&
-        resident_iterate_fits(d.mat_height, d.dia.dia_num))
-        return resident_iterate_dia(&d.dia, x, y, alpha, beta, steps, st);
-    if (d.ifusebdia && d.bdia.matinfo.height == d.mat_height && d.mat_height <= d.bdia.bdia_length_aligned &&
-        resident_iterate_fits(d.mat_height, h->bdia_ndiag))
-        return resident_iterate_bdia(&d.bdia, h->bdia_ndiag, x, y, alpha, beta, steps, st);
-    if (d.ifusecoo && h->rows.ctas) return resident_iterate_coo(&d.coo, h->rows, x, y, alpha, beta, steps, st);
-    if (d.ifusecsr && h->rows.ctas && h->csr_lanes == 0) return resident_iterate_csr(&d.csr, h->rows, x, y, alpha, beta, steps, st);
+    if (!h->resident.ctas || steps < kResidentSteps) return CLSPMV_ERR_UNSUPPORTED;
+    if (d.ifusedia) return resident_iterate_dia(&d.dia, h->resident, x, y, alpha, beta, steps, st);
+    if (d.ifusebdia) return resident_iterate_bdia(&d.bdia, h->bdia_ndiag, h->resident, x, y, alpha, beta, steps, st);
+    if (d.ifusecoo) return resident_iterate_coo(&d.coo, h->resident, x, y, alpha, beta, steps, st);
+    if (d.ifusecsr && h->csr_lanes == 0) return resident_iterate_csr(&d.csr, h->resident, x, y, alpha, beta, steps, st);
     return CLSPMV_ERR_UNSUPPORTED;
 }
 
@@ -263,8 +259,11 @@ int clspmv_cocktail_upload_f32(const clspmv_cocktail_f32* host, clspmv_cocktail_
         if (!rc) rc = cuda_status(cudaEventCreateWithFlags(&h->join[p], cudaEventDisableTiming));
     }
     if (!rc && h->nparts == 1) {
-        if (d.ifusecoo && d.coo.matinfo.height == d.mat_height) h->rows = resident_rows_plan(d.mat_height, c.coo.matinfo.nnz, c.coo.coo_row_id, nullptr);
-        if (d.ifusecsr && d.csr.matinfo.height == d.mat_height) h->rows = resident_rows_plan(d.mat_height, c.csr.matinfo.nnz, nullptr, c.csr.csr_row_ptr);
+        const int rows = d.mat_height;
+        if (d.ifusedia && d.dia.matinfo.height == rows && rows <= d.dia.dia_length_aligned) h->resident = resident_dia_plan(rows, d.dia.dia_num);
+        if (d.ifusebdia && d.bdia.matinfo.height == rows && rows <= d.bdia.bdia_length_aligned) h->resident = resident_dia_plan(rows, h->bdia_ndiag);
+        if (d.ifusecoo && d.coo.matinfo.height == rows) h->resident = resident_rows_plan(rows, c.coo.matinfo.nnz, c.coo.coo_row_id, nullptr);
+        if (d.ifusecsr && d.csr.matinfo.height == rows) h->resident = resident_rows_plan(rows, c.csr.matinfo.nnz, nullptr, c.csr.csr_row_ptr);
     }
     if (!rc) rc = cuda_status(cudaEventCreateWithFlags(&h->fork, cudaEventDisableTiming));
     if (!rc && h->nparts >= 2) {

@@ -17,9 +17,8 @@
 #include <cooperative_groups.h>
 #include <algorithm>
 #include <cstdint>
-#include <mutex>
-#include <unordered_map>
-#include <vector>
+#include <memory>
+#include <new>
 #include "api_internal.h"
 #include "clspmv_b200.h"
 
@@ -195,22 +194,19 @@ size_t smem_of(int per, int ndiag) { return sizeof(float) * (size_t)per * (ndiag
 
 size_t smem_of_rows(int per, int cap) { return sizeof(float) * ((size_t)3 * per + 1 + 2 * (size_t)cap); }
 
-// Shared memory a CTA of these kernels may ask for and its largest cluster, per device; 0 CTAs: not available.
+// Shared memory a CTA of these kernels may ask for and its largest cluster on the current device; 0 CTAs: not
+// available. Asked, with the kernels' limits raised, for each uploaded matrix (a device reset takes the raised limits back).
 struct Limits {
     size_t smem = 0;
     int ctas = 0;
 };
-Limits limits_of(int device)
+Limits raised_limits()
 {
-    static std::mutex mu;
-    static std::unordered_map<int, Limits> cache;
-    std::lock_guard<std::mutex> lock(mu);
-    auto it = cache.find(device);
-    if (it != cache.end()) return it->second;
     Limits l;
-    int optin = 0;
+    int device = 0, optin = 0;
     cudaFuncAttributes at{}, at_rows{};
-    if (cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, device) == cudaSuccess &&
+    if (cudaGetDevice(&device) == cudaSuccess &&
+        cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, device) == cudaSuccess &&
         cudaFuncGetAttributes(&at, k_dia_resident) == cudaSuccess && cudaFuncGetAttributes(&at_rows, k_rows_resident) == cudaSuccess &&
         optin > (int)std::max(at.sharedSizeBytes, at_rows.sharedSizeBytes)) {
         l.smem = (size_t)optin - std::max(at.sharedSizeBytes, at_rows.sharedSizeBytes);
@@ -236,7 +232,7 @@ Limits limits_of(int device)
         }
     }
     cudaGetLastError();
-    return cache[device] = l;
+    return l;
 }
 
 // CTAs of the cluster that holds the matrix, 0 if none does: as few as give
@@ -244,17 +240,6 @@ Limits limits_of(int device)
 // 1.4 us with 1 row per thread and 2.7 with 4 (5 diagonals, 16 CTAs), against 4.0 for a
 // launch, and 4.1 with 6: past kEntriesPerCta the launches are the faster way.
 constexpr int kEntriesPerCta = 24 * 1024;
-int ctas_for(int rows, int ndiag, int* per)
-{
-    int device = 0;
-    if (rows <= 0 || ndiag < 0 || ndiag > kMaxDiags || cudaGetDevice(&device) != cudaSuccess) return 0;
-    const Limits l = limits_of(device);
-    for (int c = 1; c <= l.ctas; c *= 2) {
-        *per = (rows + c - 1) / c;
-        if ((*per <= kThreads || c == l.ctas) && smem_of(*per, ndiag) <= l.smem && (long long)*per * ndiag <= kEntriesPerCta) return c;
-    }
-    return 0;
-}
 
 template <class K, class A>
 int launch_cluster(K kernel, const A& a, int ctas, size_t smem, cudaStream_t st)
@@ -274,44 +259,52 @@ int launch_cluster(K kernel, const A& a, int ctas, size_t smem, cudaStream_t st)
     return rc ? rc : after_launch(1);
 }
 
-int launch(const Args& in, cudaStream_t st)
+int launch(const Args& a, int ctas, cudaStream_t st)
 {
-    Args a = in;
-    const int c = ctas_for(a.rows, a.ndiag, &a.per);
-    return c ? launch_cluster(k_dia_resident, a, c, smem_of(a.per, a.ndiag), st) : CLSPMV_ERR_UNSUPPORTED;
+    return launch_cluster(k_dia_resident, a, ctas, smem_of(a.per, a.ndiag), st);
 }
 
 }  // namespace
 
-bool resident_iterate_fits(int rows, int ndiag)
+ResidentPlan resident_dia_plan(int rows, int ndiag)
 {
-    int per = 0;
-    return ctas_for(rows, ndiag, &per) > 0;
+    ResidentPlan p;
+    if (rows <= 0 || ndiag < 0 || ndiag > kMaxDiags) return p;
+    const Limits l = raised_limits();
+    for (int c = 1; c <= l.ctas; c *= 2) {
+        const int per = (rows + c - 1) / c;
+        if ((per <= kThreads || c == l.ctas) && smem_of(per, ndiag) <= l.smem && (long long)per * ndiag <= kEntriesPerCta) {
+            p.ctas = c;
+            p.per = per;
+            return p;
+        }
+    }
+    return p;
 }
 
-int resident_iterate_dia(const clspmv_dia_f32* m, float* x, float* y, float alpha, float beta, int steps, cudaStream_t st)
+int resident_iterate_dia(const clspmv_dia_f32* m, const ResidentPlan& p, float* x, float* y, float alpha, float beta, int steps, cudaStream_t st)
 {
-    return launch(Args{m->matinfo.height, m->matinfo.width, m->dia_num, 0, m->dia_length_aligned, m->dia_offsets, nullptr, 0,
-                       m->dia_data, x, y, alpha, beta, steps}, st);
+    return launch(Args{m->matinfo.height, m->matinfo.width, m->dia_num, p.per, m->dia_length_aligned, m->dia_offsets, nullptr, 0,
+                       m->dia_data, x, y, alpha, beta, steps}, p.ctas, st);
 }
 
-int resident_iterate_bdia(const clspmv_bdia_f32* m, int ndiag, float* x, float* y, float alpha, float beta, int steps, cudaStream_t st)
+int resident_iterate_bdia(const clspmv_bdia_f32* m, int ndiag, const ResidentPlan& p, float* x, float* y, float alpha, float beta, int steps,
+                          cudaStream_t st)
 {
-    return launch(Args{m->matinfo.height, m->matinfo.width, ndiag, 0, m->bdia_length_aligned, m->bdia_offsets, m->bdia_bptr,
-                       m->bdia_band_num, m->bdia_data, x, y, alpha, beta, steps}, st);
+    return launch(Args{m->matinfo.height, m->matinfo.width, ndiag, p.per, m->bdia_length_aligned, m->bdia_offsets, m->bdia_bptr,
+                       m->bdia_band_num, m->bdia_data, x, y, alpha, beta, steps}, p.ctas, st);
 }
 
 // Rows longer than this keep one thread too long; they stay with the launches.
 constexpr int kLongestRow = 64;
 
-ResidentRows resident_rows_plan(int rows, int nnz, const int* row_id, const int* row_ptr)
+ResidentPlan resident_rows_plan(int rows, int nnz, const int* row_id, const int* row_ptr)
 {
-    ResidentRows p;
-    int device = 0;
-    if (rows <= 0 || nnz < 0 || (nnz > 0 && !row_id && !row_ptr) || nnz > kMaxCtas * kEntriesPerCta || rows > kMaxCtas * kEntriesPerCta ||
-        cudaGetDevice(&device) != cudaSuccess)
+    ResidentPlan p;
+    if (rows <= 0 || nnz < 0 || (nnz > 0 && !row_id && !row_ptr) || nnz > kMaxCtas * kEntriesPerCta || rows > kMaxCtas * kEntriesPerCta)
         return p;
-    std::vector<int> ptr((size_t)rows + 1, 0);
+    const std::unique_ptr<int[]> ptr(new (std::nothrow) int[(size_t)rows + 1]());
+    if (!ptr) return p;
     if (row_id) {
         for (int i = 0; i < nnz; i++) {
             if (row_id[i] < 0 || row_id[i] >= rows || (i > 0 && row_id[i] < row_id[i - 1])) return p;
@@ -319,11 +312,11 @@ ResidentRows resident_rows_plan(int rows, int nnz, const int* row_id, const int*
         }
         for (int r = 0; r < rows; r++) ptr[(size_t)r + 1] += ptr[(size_t)r];
     } else {
-        std::copy(row_ptr, row_ptr + rows + 1, ptr.begin());
+        std::copy(row_ptr, row_ptr + rows + 1, ptr.get());
     }
     for (int r = 0; r < rows; r++)
         if (ptr[(size_t)r + 1] < ptr[(size_t)r] || ptr[(size_t)r + 1] - ptr[(size_t)r] > kLongestRow) return p;
-    const Limits l = limits_of(device);
+    const Limits l = raised_limits();
     for (int c = 1; c <= l.ctas; c *= 2) {
         const int per = (rows + c - 1) / c;
         int cap = 0;
@@ -338,13 +331,13 @@ ResidentRows resident_rows_plan(int rows, int nnz, const int* row_id, const int*
     return p;
 }
 
-int resident_iterate_coo(const clspmv_coo_f32* m, const ResidentRows& p, float* x, float* y, float alpha, float beta, int steps, cudaStream_t st)
+int resident_iterate_coo(const clspmv_coo_f32* m, const ResidentPlan& p, float* x, float* y, float alpha, float beta, int steps, cudaStream_t st)
 {
     return launch_cluster(k_rows_resident, RowArgs{m->matinfo.height, m->matinfo.width, m->matinfo.nnz, p.per, p.cap, m->coo_row_id, nullptr,
                                                    m->coo_col_id, m->coo_data, x, y, alpha, beta, steps}, p.ctas, smem_of_rows(p.per, p.cap), st);
 }
 
-int resident_iterate_csr(const clspmv_csr_f32* m, const ResidentRows& p, float* x, float* y, float alpha, float beta, int steps, cudaStream_t st)
+int resident_iterate_csr(const clspmv_csr_f32* m, const ResidentPlan& p, float* x, float* y, float alpha, float beta, int steps, cudaStream_t st)
 {
     return launch_cluster(k_rows_resident, RowArgs{m->matinfo.height, m->matinfo.width, m->matinfo.nnz, p.per, p.cap, nullptr, m->csr_row_ptr,
                                                    m->csr_col_id, m->csr_data, x, y, alpha, beta, steps}, p.ctas, smem_of_rows(p.per, p.cap), st);
