@@ -572,7 +572,7 @@ __global__ void __launch_bounds__(kSpmmBlock) k_spmm_warp_rows(int rows, const i
 //
 // A CSR row that starts and ends in its warp's run is written directly
 // (alpha, beta), its pieces in several slots summed by a segmented scan, so
-// Y gets no scaling pass of its own. Only rows cut by an edge between warps
+// Y gets no scaling pass of its own (ADD: for beta = 1 it is added). Only rows cut by an edge between warps
 // are added atomically, after k_scale_cut has applied beta to those and to
 // the rows without entries. COO has no row pointer to tell them by: beta is
 // applied to all of Y first and every row is added, by red.global.add, which
@@ -737,7 +737,7 @@ __device__ __forceinline__ float4 shfl_up_x(float4 v, int o) { return f4up(v, o)
 __device__ __forceinline__ float x_add(float a, float b) { return a + b; }
 __device__ __forceinline__ float4 x_add(float4 a, float4 b) { return f4add(a, b); }
 
-template <int LG, int VEC, int P, class T, bool IS_CSR>
+template <int LG, int VEC, int P, class T, bool IS_CSR, bool ADD>
 __global__ void __launch_bounds__(kSpmmBlock, 4) k_spmm_runs(int rows, int nnz, const int* __restrict__ row_ptr,
                                                              const int* __restrict__ row_id, const int* __restrict__ col_id,
                                                              const T* __restrict__ vals, bool vec, int per, Dense d)
@@ -789,7 +789,7 @@ __global__ void __launch_bounds__(kSpmmBlock, 4) k_spmm_runs(int rows, int nnz, 
             float a = d.alpha;
             if (!std::is_same<T, float>::value) a *= d.scale[r];
             float* y = Y + (size_t)r * d.ldy;
-            if (!IS_CSR || !whole) s.atomic(y, a);
+            if (ADD || !whole) s.atomic(y, a);
             else if (VEC == 1) s.store_cs(y, a, d.beta);
             else s.store(y, a, d.beta);
         };
@@ -1063,14 +1063,15 @@ bool warp_rows_enabled()
 }
 
 template <int LG, int VEC, int P, class T, bool IS_CSR>
-void launch_runs(int rows, int nnz, const int* row_ptr, const int* row_id, const int* col_id, const T* v, bool vec, Dense d,
-                 cudaStream_t st)
+void launch_runs(int rows, int nnz, const int* row_ptr, const int* row_id, const int* col_id, const T* v, bool vec, bool add,
+                 Dense d, cudaStream_t st)
 {
     const long long runs = ((long long)nnz + 32 * P - 1) / (32 * P), wpb = kSpmmBlock / 32;
     const long long resident = 148LL * 4 * wpb;
     const long long per = (runs + resident - 1) / resident;   // 1 while the runs do not fill the device
     const int grid = (int)((runs + per * wpb - 1) / (per * wpb));
-    k_spmm_runs<LG, VEC, P, T, IS_CSR><<<grid, kSpmmBlock, 0, st>>>(rows, nnz, row_ptr, row_id, col_id, v, vec, (int)per, d);
+    if (!IS_CSR || add) k_spmm_runs<LG, VEC, P, T, IS_CSR, true><<<grid, kSpmmBlock, 0, st>>>(rows, nnz, row_ptr, row_id, col_id, v, vec, (int)per, d);
+    else k_spmm_runs<LG, VEC, P, T, IS_CSR, !IS_CSR><<<grid, kSpmmBlock, 0, st>>>(rows, nnz, row_ptr, row_id, col_id, v, vec, (int)per, d);
 }
 
 template <class T, bool IS_CSR>
@@ -1080,8 +1081,14 @@ int launch_chunks(int rows, int nnz, const int* row_ptr, const int* row_id, cons
     // 8 nonzeros per lane from where their runs fill the device's warps (1.2M nonzeros): 4 loses up to 1.4x there
     // at k <= 16 (more searches and scans a nonzero) and wins 1.1-1.4x on 0.24M nonzeros (more warps)
     const bool few = nnz < 148 * 32 * 256;
+    // A CSR row is added, not written, where Y holds beta * Y already: a row that reads its Y first waits for it, one
+    // row after another in a slot. beta = 1, us written / added: 5,000 rows of 3 at k = 36 27 / 14, 2^20 rows of 2 at
+    // k = 5 / 36 / 128 45 / 33, 157 / 125, 355 / 343. Other beta than 0 take a pass over Y for that, which pays for
+    // single columns (k < 8 or rows off 16 bytes) of a small Y: 200,000 rows of 9 at k = 5 47 / 35, 20,000 18 / 15,
+    // but 2^20 rows of 2 51 / 54, and at k = 16 60,000 rows 12.8 / 16.9.
+    const bool add = d.beta == 1.0f || (d.beta != 0.0f && vec == 1 && (long long)rows * d.k <= 1 << 20);
     if (d.beta != 1.0f) {
-        if (IS_CSR && nnz > 0)
+        if (IS_CSR && nnz > 0 && !add)
             (vec == 4 ? k_scale_cut<4> : k_scale_cut<1>)<<<grid_of(rows), kSpmmBlock, 0, st>>>(
                 rows, row_ptr, few ? 128 : 256, vec == 1 && d.k < 8 ? 0 : d.lshift, d);
         else
@@ -1094,8 +1101,8 @@ int launch_chunks(int rows, int nnz, const int* row_ptr, const int* row_id, cons
     const bool al = ((uintptr_t)col_id & 15) == 0 && (IS_CSR || ((uintptr_t)row_id & 15) == 0) && ((uintptr_t)v & (4 * sizeof(T) - 1)) == 0;
 #define RUNS(LG, VEC)                                                                                            \
     case LG:                                                                                                     \
-        if (few) launch_runs<LG, VEC, 4, T, IS_CSR>(rows, nnz, row_ptr, row_id, col_id, v, al, d, st);           \
-        else launch_runs<LG, VEC, 8, T, IS_CSR>(rows, nnz, row_ptr, row_id, col_id, v, al, d, st);               \
+        if (few) launch_runs<LG, VEC, 4, T, IS_CSR>(rows, nnz, row_ptr, row_id, col_id, v, al, add, d, st);           \
+        else launch_runs<LG, VEC, 8, T, IS_CSR>(rows, nnz, row_ptr, row_id, col_id, v, al, add, d, st);               \
         break;
     if (vec == 4) {
         switch (d.lshift) {

@@ -78,3 +78,9 @@ def test_empty_rows_are_written_in_lines():
     """9 of 10 rows empty at k = 128: beta = 0, which has to write them, took 8.8 times as long as beta = 1, which does not."""
     m = _device(1 << 20, 0.1, 8)
     assert _us(m, 128, 0.0) <= 4 * _us(m, 128, 1.0)
+
+
+def test_rows_do_not_wait_for_their_y():
+    """2^20 rows of 2 at k = 36: beta = 1, without a pass of its own, took 1.31 times as long as beta = 0."""
+    m = _device(1 << 20, 1, 2)
+    assert _us(m, 36, 1.0) <= 1.15 * _us(m, 36, 0.0)
