@@ -565,7 +565,8 @@ __global__ void __launch_bounds__(kSpmmBlock) k_spmm_warp_rows(int rows, const i
 // CSR / COO by warp runs. A warp takes 32 P consecutive nonzeros, P per lane
 // with 128-bit loads, finds the row of each (CSR: from row_ptr), and splits
 // its lanes into slots of G = 2^LG lanes that share the k columns of X and Y
-// (VEC columns a lane). A slot owns the P G nonzeros that its lanes loaded
+// (VEC columns a lane), or those of the block's panel (blockIdx.y) where few
+// nonzeros are worth more warps than that. A slot owns the P G nonzeros that its lanes loaded
 // and hands them round by shuffles, with kRunLoads X rows in flight: ids,
 // values and rows are read once, coalesced, and no lane waits for row_ptr
 // between two nonzeros.
@@ -607,6 +608,12 @@ __global__ void __launch_bounds__(kSpmmBlock) k_scale_cut(int rows, const int* _
             const int s = __ldg(row_ptr + r0 + lane), e = __ldg(row_ptr + r0 + lane + 1);
             need = s >= e || s / run != (e - 1) / run;
         }
+        if (VEC == 1 && lshift == 0) {
+            float* y = d.Y + (size_t)(r0 + lane) * d.ldy;
+            if (need)
+                for (int j = 0; j < d.k; j++) y[j] = d.beta == 0.0f ? 0.0f : d.beta * y[j];
+            continue;
+        }
         const unsigned mask = __ballot_sync(kWarpAll, need);
         if (!mask) continue;
 #pragma unroll 4
@@ -614,7 +621,6 @@ __global__ void __launch_bounds__(kSpmmBlock) k_scale_cut(int rows, const int* _
             if (!(mask >> i & slots)) continue;
             if (!(mask >> (i + slot) & 1)) continue;
             float* y = d.Y + (size_t)(r0 + i + slot) * d.ldy;
-#pragma unroll 4
             for (int c = c0; c < d.k; c += G * VEC) {
                 if (VEC == 4) {
                     float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
@@ -746,7 +752,7 @@ __global__ void __launch_bounds__(kSpmmBlock, 4) k_spmm_runs(int rows, int nnz, 
     static_assert(P % U == 0, "a batch of X rows stays within a lane's nonzeros");
     using XT = typename Acc<VEC>::X;
     const int lane = threadIdx.x & 31, slot = lane >> LG;
-    const int c0 = (lane & (G - 1)) * VEC;
+    const int c0 = ((int)blockIdx.y * G + (lane & (G - 1))) * VEC;
     const bool cols = c0 < d.k;
     const float* __restrict__ X = d.X + (cols ? c0 : 0);
     float* const Y = d.Y + c0;
@@ -1069,7 +1075,7 @@ void launch_runs(int rows, int nnz, const int* row_ptr, const int* row_id, const
     const long long runs = ((long long)nnz + 32 * P - 1) / (32 * P), wpb = kSpmmBlock / 32;
     const long long resident = 148LL * 4 * wpb;
     const long long per = (runs + resident - 1) / resident;   // 1 while the runs do not fill the device
-    const int grid = (int)((runs + per * wpb - 1) / (per * wpb));
+    const dim3 grid((unsigned)((runs + per * wpb - 1) / (per * wpb)), (unsigned)((d.k + (VEC << LG) - 1) / (VEC << LG)));
     if (!IS_CSR || add) k_spmm_runs<LG, VEC, P, T, IS_CSR, true><<<grid, kSpmmBlock, 0, st>>>(rows, nnz, row_ptr, row_id, col_id, v, vec, (int)per, d);
     else k_spmm_runs<LG, VEC, P, T, IS_CSR, !IS_CSR><<<grid, kSpmmBlock, 0, st>>>(rows, nnz, row_ptr, row_id, col_id, v, vec, (int)per, d);
 }
@@ -1081,6 +1087,13 @@ int launch_chunks(int rows, int nnz, const int* row_ptr, const int* row_id, cons
     // 8 nonzeros per lane from where their runs fill the device's warps (1.2M nonzeros): 4 loses up to 1.4x there
     // at k <= 16 (more searches and scans a nonzero) and wins 1.1-1.4x on 0.24M nonzeros (more warps)
     const bool few = nnz < 148 * 32 * 256;
+    // Few nonzeros leave warps idle while a slot of G lanes walks its 4 G nonzeros: G is halved, down to 4 lanes, until the
+    // panels of G lanes' columns make 3/8 of the device's warps (all of them: 20,000 rows of 9 at k = 64 17 -> 19 us; down to 2
+    // lanes: 3,000 rows of 4 at k = 12 15 -> 21). beta 0, us: 5,000 rows of 3 at k = 36 / 128 19 / 23 -> 13 / 13 (at beta 1
+    // 14 / 19 -> 8 / 8), 60,000 rows of 2 17 / 23 -> 15 / 19, 20,000 rows of 9 19 / 25 -> 17 / 21.
+    int lg = d.lshift;
+    if (few)
+        while (lg > 2 && ((long long)nnz + 127) / 128 * ((d.k + (vec << lg) - 1) / (vec << lg)) < 148 * 12) lg--;
     // A CSR row is added, not written, where Y holds beta * Y already: a row that reads its Y first waits for it, one
     // row after another in a slot. beta = 1, us written / added: 5,000 rows of 3 at k = 36 27 / 14, 2^20 rows of 2 at
     // k = 5 / 36 / 128 45 / 33, 157 / 125, 355 / 343. Other beta than 0 take a pass over Y for that, which pays for
@@ -1105,11 +1118,11 @@ int launch_chunks(int rows, int nnz, const int* row_ptr, const int* row_id, cons
         else launch_runs<LG, VEC, 8, T, IS_CSR>(rows, nnz, row_ptr, row_id, col_id, v, al, add, d, st);               \
         break;
     if (vec == 4) {
-        switch (d.lshift) {
+        switch (lg) {
             RUNS(0, 4) RUNS(1, 4) RUNS(2, 4) RUNS(3, 4) RUNS(4, 4) RUNS(5, 4)
         }
     } else {
-        switch (d.lshift) {
+        switch (lg) {
             RUNS(0, 1) RUNS(1, 1) RUNS(2, 1) RUNS(3, 1) RUNS(4, 1) RUNS(5, 1)
         }
     }

@@ -84,3 +84,9 @@ def test_rows_do_not_wait_for_their_y():
     """2^20 rows of 2 at k = 36: beta = 1, without a pass of its own, took 1.31 times as long as beta = 0."""
     m = _device(1 << 20, 1, 2)
     assert _us(m, 36, 1.0) <= 1.15 * _us(m, 36, 0.0)
+
+
+def test_few_nonzeros_take_more_warps():
+    """5,000 rows of 3: k = 128 took 1.8 times as long as k = 16."""
+    m = _device(5000, 1, 3)
+    assert _us(m, 128, 0.0) <= 1.45 * _us(m, 16, 0.0)
