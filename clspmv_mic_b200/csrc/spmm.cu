@@ -1362,11 +1362,10 @@ __device__ __forceinline__ void batch_chunk(const BatchJob& J, int e0, int c0)
     flush(true);
 }
 
-// OCC CTAs per SM: 4 at the 64 registers of the row walks, 6 at 40, which
-// spills around the dispatch but has half as many X lookups again in flight.
-// Which one a batch takes: prefers_wide.
-template <int OCC>
-__global__ void __launch_bounds__(kSpmmBlock, OCC) k_batch(const BatchJob* __restrict__ jobs, int njobs, long long tasks)
+// 4 CTAs per SM, at 64 registers: without the bound a lane group takes 1.2 times as long over a long row (ten rows of
+// 20,000 at k = 4: 1.70 against 1.39 ms). 6 CTAs, at 40, leave one lookup in flight: SELL rows of 20,000 at k = 1 1.2
+// against 2.7 ms, at k = 32 2.1 against 3.3, for 4 to 13 % in batches of even rows at k = 1, 16 and 32.
+__global__ void __launch_bounds__(kSpmmBlock, 4) k_batch(const BatchJob* __restrict__ jobs, int njobs, long long tasks)
 {
     const int lane = threadIdx.x & 31;
     const long long nwarps = ((long long)gridDim.x * kSpmmBlock) >> 5;
@@ -1453,39 +1452,10 @@ int batch_blocks_grid()
     return persistent_grid((const void*)k_batch_blocks, &grid);
 }
 
-// X of a row job whose rows take several lanes on 16-byte slices (k = 8, 12, ...), else 0.
-long long x_bytes_of_lane_groups(const BatchJob& J)
+int batch_grid()
 {
-    return J.vec == 4 && J.lshift > 0 && !J.chunk ? 4LL * J.k * J.m.csr.matinfo.width : 0;
-}
-
-// Whether a row job gains from 6 CTAs per SM. us of whole batches, 4 against
-// 6 CTAs: 48 uneven matrices (5-32 nonzeros a row, up to 500k rows, 41M in
-// all) at k = 1 362 / 348, k = 4 363 / 383, k = 8 474 / 445, k = 16 733 / 634,
-// k = 32 1311 / 1098, k = 64 2803 / 2467; 14 of up to 225k rows at k = 1
-// 20.7 / 19.1, k = 8 32.9 / 32.9, k = 16 43.3 / 44.6, k = 32 80 / 74. So: one
-// column, or 8 and more lanes a row; 2-7 lanes where the X read that way
-// passes half of L2, one die's share (66-88 MB at k = 8 of the first batch, 20
-// MB at k = 16 of the second: lookups that hit are short enough for 4 CTAs);
-// not at k = 4, where the lookups fill L1 as it is, nor for chunk jobs and
-// other k that read X by single floats, which were not measured to gain.
-constexpr long long kBatchX = 63LL << 20;
-bool prefers_wide(const BatchJob& J, long long multi_x)
-{
-    if (J.chunk) return false;
-    if (J.vec != 4) return J.k == 1;
-    return J.lshift >= 3 || (J.lshift > 0 && multi_x > kBatchX);
-}
-
-constexpr int kBatchOccNarrow = 4, kBatchOccWide = 6;
-
-template <int OCC>
-int launch_rows(const BatchJob* jobs, int njobs, long long tasks, cudaStream_t st)
-{
-    static int cache = 0;
-    const long long grid = std::min<long long>(persistent_grid((const void*)k_batch<OCC>, &cache), (tasks + 7) / 8);
-    k_batch<OCC><<<(int)grid, kSpmmBlock, 0, st>>>(jobs, njobs, tasks);
-    return 1;
+    static int grid = 0;
+    return persistent_grid((const void*)k_batch, &grid);
 }
 
 // Fills one device job from a caller's job description.
@@ -1553,7 +1523,6 @@ struct clspmv_batch {
     int nrow_jobs = 0;            // jobs [0, nrow_jobs) run in k_batch, the rest (4x4 blocks) in k_batch_blocks
     long long tasks = 0;
     long long block_tasks = 0;
-    bool wide = false;            // most row tasks gain from 6 CTAs per SM (prefers_wide)
     BatchJob* host = nullptr;     // pinned staging of the job table
     BatchJob* dev = nullptr;
     cudaEvent_t copied = nullptr; // the last table upload has left `host`
@@ -1700,19 +1669,15 @@ int clspmv_batch_set(clspmv_batch* b, const clspmv_spmm_job* jobs, int njobs, cl
         else b->host[b->nrow_jobs++] = J;
     }
     std::reverse(b->host + b->nrow_jobs, b->host + njobs);
-    long long tasks = 0, block_tasks = 0, wide_tasks = 0, multi_x = 0;
-    for (int i = 0; i < b->nrow_jobs; i++) multi_x += x_bytes_of_lane_groups(b->host[i]);
+    long long tasks = 0, block_tasks = 0;
     for (int i = 0; i < njobs; i++) {
         BatchJob& J = b->host[i];
         long long& t = J.bh ? block_tasks : tasks;
         J.task_begin = t;
         const long long units = J.chunk > 0 ? ((long long)J.nnz + J.chunk - 1) / J.chunk
                                 : J.bh ? ((long long)J.rows + J.bh - 1) / J.bh : J.rows;
-        const long long n = (units + (32 >> J.lshift) - 1) / (32 >> J.lshift);
-        t += n;
-        if (!J.bh && prefers_wide(J, multi_x)) wide_tasks += n;
+        t += (units + (32 >> J.lshift) - 1) / (32 >> J.lshift);
     }
-    b->wide = 2 * wide_tasks > tasks;
     b->njobs = njobs;
     b->tasks = tasks;
     b->block_tasks = block_tasks;
@@ -1728,8 +1693,9 @@ int clspmv_batch_run(clspmv_batch* b, clspmv_stream_t stream)
     cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);
     int n = 0;
     if (b->tasks > 0) {
-        n += b->wide ? launch_rows<kBatchOccWide>(b->dev, b->nrow_jobs, b->tasks, st)
-                     : launch_rows<kBatchOccNarrow>(b->dev, b->nrow_jobs, b->tasks, st);
+        const long long grid = std::min<long long>(batch_grid(), (b->tasks + 7) / 8);
+        k_batch<<<(int)grid, kSpmmBlock, 0, st>>>(b->dev, b->nrow_jobs, b->tasks);
+        n++;
     }
     if (b->block_tasks > 0) {
         const long long grid = std::min<long long>(batch_blocks_grid(), (b->block_tasks + 7) / 8);
