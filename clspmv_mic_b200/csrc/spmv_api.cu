@@ -1204,6 +1204,7 @@ int clspmv_sell_plan_create(const clspmv_sell_f32* m, clspmv_sell_plan** out)
         // reads the tails' column ids in place (for measurements)
         const char* e = getenv("CLSPMV_SELL_SPLIT");
         p->split = !(e && atoi(e) == 0);
+        if (!p->split) p->even = 0;
         const char* tcmp = getenv("CLSPMV_SELL_TAIL_COMPACT");
         p->compact = !(tcmp && atoi(tcmp) == 0);
     }
