@@ -591,13 +591,13 @@ __global__ void __launch_bounds__(kSpmmBlock) k_spmm_warp_rows(int rows, const i
 // ---------------------------------------------------------------------------
 constexpr int kRunLoads = 4;
 
-// beta to the rows that an edge between warp runs of `run` nonzeros cuts, and to rows without entries: a warp looks at
+// beta to the rows that an edge between warp runs of 2^lrun nonzeros cuts, and to rows without entries: a warp looks at
 // 32 rows, a lane each, and groups of 2^lshift lanes write the ones that need it. A thread per row at every k wrote 32
 // lines a store: with 9 of 10 of 2^20 rows empty 872 us of a product at k = 128, 433 at k = 64, 100 at k = 16 (beta 0),
 // against 178, 104 and 48. It stays for fewer than 8 single columns (lshift 0: 4M rows, 1 of 50 with entries, k = 5: 61
 // us, 70 with 8 lanes a row).
 template <int VEC>
-__global__ void __launch_bounds__(kSpmmBlock) k_scale_cut(int rows, const int* __restrict__ row_ptr, int run, int lshift, Dense d)
+__global__ void __launch_bounds__(kSpmmBlock) k_scale_cut(int rows, const int* __restrict__ row_ptr, int lrun, int lshift, Dense d)
 {
     const int lane = threadIdx.x & 31, G = 1 << lshift, slot = lane >> lshift, c0 = (lane & (G - 1)) * VEC;
     const unsigned slots = lshift == 0 ? kWarpAll : (1u << (32 >> lshift)) - 1;
@@ -606,7 +606,7 @@ __global__ void __launch_bounds__(kSpmmBlock) k_scale_cut(int rows, const int* _
         bool need = false;
         if (r0 + lane < rows) {
             const int s = __ldg(row_ptr + r0 + lane), e = __ldg(row_ptr + r0 + lane + 1);
-            need = s >= e || s / run != (e - 1) / run;
+            need = s >= e || s >> lrun != (e - 1) >> lrun;
         }
         if (VEC == 1 && lshift == 0) {
             float* y = d.Y + (size_t)(r0 + lane) * d.ldy;
@@ -1103,7 +1103,7 @@ int launch_chunks(int rows, int nnz, const int* row_ptr, const int* row_id, cons
     if (d.beta != 1.0f) {
         if (IS_CSR && nnz > 0 && !add)
             (vec == 4 ? k_scale_cut<4> : k_scale_cut<1>)<<<grid_of(rows), kSpmmBlock, 0, st>>>(
-                rows, row_ptr, few ? 128 : 256, vec == 1 && d.k < 8 ? 0 : d.lshift, d);
+                rows, row_ptr, few ? 7 : 8, vec == 1 && d.k < 8 ? 0 : d.lshift, d);
         else
             k_scale_rows<<<grid_of((long long)rows * d.k), kSpmmBlock, 0, st>>>(d.Y, rows, d.k, d.ldy, d.beta);
         int rc = after_launch(1);
