@@ -51,11 +51,12 @@ int launch_diag_bulk(int rows, int cols, int ndiag, int len, const int* offsets,
 // memory, in one launch (iterate_resident.cu); x holds at least as many entries as y.
 // The plans are made where the matrix is uploaded, with its device current.
 struct ResidentPlan {
-    int ctas = 0, per = 0, cap = 0;   // CTAs of the cluster (0: the matrix does not fit), rows and most entries of one (COO, CSR)
+    int ctas = 0, per = 0, cap = 0;   // CTAs of the cluster (0: the matrix does not fit, or gains nothing), rows and most entries of one (COO, CSR)
 };
 ResidentPlan resident_dia_plan(int rows, int ndiag);
+ResidentPlan resident_bdia_plan(int rows, const int* bptr, int nband);
 // COO (sorted row ids) or CSR (row pointer), from the host arrays.
-ResidentPlan resident_rows_plan(int rows, int nnz, const int* row_id, const int* row_ptr);
+ResidentPlan resident_rows_plan(int rows, int nnz, const int* row_id, const int* row_ptr, const int* col);
 int resident_iterate_dia(const clspmv_dia_f32* m, const ResidentPlan& p, float* x, float* y, float alpha, float beta, int steps, cudaStream_t st);
 int resident_iterate_bdia(const clspmv_bdia_f32* m, int ndiag, const ResidentPlan& p, float* x, float* y, float alpha, float beta, int steps,
                           cudaStream_t st);

@@ -261,9 +261,9 @@ int clspmv_cocktail_upload_f32(const clspmv_cocktail_f32* host, clspmv_cocktail_
     if (!rc && h->nparts == 1) {
         const int rows = d.mat_height;
         if (d.ifusedia && d.dia.matinfo.height == rows && rows <= d.dia.dia_length_aligned) h->resident = resident_dia_plan(rows, d.dia.dia_num);
-        if (d.ifusebdia && d.bdia.matinfo.height == rows && rows <= d.bdia.bdia_length_aligned) h->resident = resident_dia_plan(rows, h->bdia_ndiag);
-        if (d.ifusecoo && d.coo.matinfo.height == rows) h->resident = resident_rows_plan(rows, c.coo.matinfo.nnz, c.coo.coo_row_id, nullptr);
-        if (d.ifusecsr && d.csr.matinfo.height == rows) h->resident = resident_rows_plan(rows, c.csr.matinfo.nnz, nullptr, c.csr.csr_row_ptr);
+        if (d.ifusebdia && d.bdia.matinfo.height == rows && rows <= d.bdia.bdia_length_aligned) h->resident = resident_bdia_plan(rows, c.bdia.bdia_bptr, c.bdia.bdia_band_num);
+        if (d.ifusecoo && d.coo.matinfo.height == rows) h->resident = resident_rows_plan(rows, c.coo.matinfo.nnz, c.coo.coo_row_id, nullptr, c.coo.coo_col_id);
+        if (d.ifusecsr && d.csr.matinfo.height == rows) h->resident = resident_rows_plan(rows, c.csr.matinfo.nnz, nullptr, c.csr.csr_row_ptr, c.csr.csr_col_id);
     }
     if (!rc) rc = cuda_status(cudaEventCreateWithFlags(&h->fork, cudaEventDisableTiming));
     if (!rc && h->nparts >= 2) {

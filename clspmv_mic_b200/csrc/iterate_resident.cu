@@ -8,7 +8,7 @@
 // part, twice (the last result and the next one). A row's entries that lie in
 // another run are read from its owner's shared memory (ld.shared::cluster),
 // and one cluster barrier ends a step: all reads of the old vector are done
-// before anybody writes over it in the step after the next. Rows are summed
+// before anybody writes over it in the next step. Rows are summed
 // by one thread each, in stored order.
 //
 // 40 steps on one B200, a copy and a launch per step / a launch per step /
@@ -29,7 +29,7 @@ namespace {
 
 constexpr int kThreads = 1024;
 constexpr int kMaxCtas = 16;       // a cluster above 8 CTAs is opt-in
-constexpr int kMaxDiags = 256;
+constexpr int kMaxDiags = 128;
 
 struct Args {
     int rows, cols, ndiag, per;    // per: rows of a CTA
@@ -266,6 +266,21 @@ int launch(const Args& a, int ctas, cudaStream_t st)
 
 }  // namespace
 
+// A resident step takes 1.2 us and 0.15 us a diagonal (a run's edge reads it
+// from another CTA), a launch's 3.3 us and 0.18 us a diagonal for DIA, 0.31
+// us per 4 diagonals of a band for BDIA. So DIA stays to kMaxDiags (150
+// diagonals at 2,000 rows, 4 / 40 steps: 33.2 / 31.3 us a step by launches, 33.5 / 23.0
+// resident; 250 at 1,200 rows 49 / 48 and 69 / 52), BDIA while diagonals are few for
+// their bands (one band of 24, 31, 64 at 2,000 rows, 16 steps: 5.1, 5.7, 8.6
+// and 5.1, 6.0, 11.1; nine bands of 3 at 8,000 rows 6.6 and 6.5).
+ResidentPlan resident_bdia_plan(int rows, const int* bptr, int nband)
+{
+    long long quads = 0;
+    for (int b = 0; b < nband; b++) quads += (bptr[b + 1] - bptr[b] + 3) / 4;
+    const int ndiag = nband > 0 ? bptr[nband] : 0;
+    return ndiag <= 11 + 2 * quads ? resident_dia_plan(rows, ndiag) : ResidentPlan{};
+}
+
 ResidentPlan resident_dia_plan(int rows, int ndiag)
 {
     ResidentPlan p;
@@ -298,10 +313,52 @@ int resident_iterate_bdia(const clspmv_bdia_f32* m, int ndiag, const ResidentPla
 // Rows longer than this keep one thread too long; they stay with the launches.
 constexpr int kLongestRow = 64;
 
-ResidentPlan resident_rows_plan(int rows, int nnz, const int* row_id, const int* row_ptr)
+// us of a step of one CTA's rows [b, b + n): the barrier, the accesses to its
+// own shared memory (a warp's lanes start at their rows' first entries: g of
+// them in one bank take g turns), the chain of the longest row of each pass,
+// and the reads of other CTAs, whose time goes with the CTAs that a warp's
+// lanes read from at once. Fitted to 246 matrices of 200 to 46,000 rows
+// (stencils, bands, rows of up to 60 columns near the diagonal or anywhere)
+// at 40 steps on B200, 9 % off on average; the chain's share is then taken a
+// third higher, which keeps rows of over 30 entries, the ones off by more
+// (up to 28 %), on the safe side. CTAs of several passes are estimated from
+// every fourth warp, 0.2 ms of an upload of 330k entries.
+double rows_step_us(const int* ptr, const int* col, int rows, int per, int b)
+{
+    const int n = std::min(per, rows - b), skip = n > kThreads ? 4 : 1;
+    double turns = 0, slots = 0, chain = 0, others = 0;
+    for (int p0 = 0; p0 < n; p0 += kThreads) {
+        int pass = 0;
+        for (int w0 = p0; w0 < std::min(n, p0 + kThreads); w0 += 32 * skip) {
+            const int lanes = std::min(32, n - w0);
+            int bank[32] = {}, g = 0, longest = 0;
+            unsigned owners[kLongestRow] = {};   // CTAs that the lanes read entry j from; bit 16: past the rows, in global memory
+            for (int r = b + w0; r < b + w0 + lanes; r++) {
+                const int first = ptr[r], len = ptr[r + 1] - first;
+                g = std::max(g, ++bank[(first - ptr[b]) & 31]);
+                longest = std::max(longest, len);
+                for (int j = 0; j < len; j++) {
+                    const int c = col[first + j];
+                    if ((unsigned)(c - b) >= (unsigned)per) owners[j] |= 1u << (c < rows ? c / per : kMaxCtas);
+                }
+            }
+            for (int j = 0; j < longest; j++) others += __builtin_popcount(owners[j]);
+            turns += (double)longest * g;
+            slots += longest;
+            pass = std::max(pass, longest);
+        }
+        chain += pass;
+    }
+    return 0.7 + 0.055 * chain + skip * (0.0008 * turns + 0.0016 * slots + 0.0065 * others);
+}
+
+// A little under what a step by launches takes, replayed: COO's two 4.2-5.8 us, CSR's 5.6-8.3.
+constexpr double kCooStep = 4.0, kCsrStep = 5.0;
+
+ResidentPlan resident_rows_plan(int rows, int nnz, const int* row_id, const int* row_ptr, const int* col)
 {
     ResidentPlan p;
-    if (rows <= 0 || nnz < 0 || (nnz > 0 && !row_id && !row_ptr) || nnz > kMaxCtas * kEntriesPerCta || rows > kMaxCtas * kEntriesPerCta)
+    if (rows <= 0 || nnz < 0 || (nnz > 0 && ((!row_id && !row_ptr) || !col)) || nnz > kMaxCtas * kEntriesPerCta || rows > kMaxCtas * kEntriesPerCta)
         return p;
     const std::unique_ptr<int[]> ptr(new (std::nothrow) int[(size_t)rows + 1]());
     if (!ptr) return p;
@@ -314,6 +371,9 @@ ResidentPlan resident_rows_plan(int rows, int nnz, const int* row_id, const int*
     } else {
         std::copy(row_ptr, row_ptr + rows + 1, ptr.get());
     }
+    int sign = 0;
+    for (int i = 0; i < nnz; i++) sign |= col[i];
+    if (sign < 0 || ptr[0] != 0 || ptr[(size_t)rows] > nnz) return p;
     for (int r = 0; r < rows; r++)
         if (ptr[(size_t)r + 1] < ptr[(size_t)r] || ptr[(size_t)r + 1] - ptr[(size_t)r] > kLongestRow) return p;
     const Limits l = raised_limits();
@@ -322,6 +382,8 @@ ResidentPlan resident_rows_plan(int rows, int nnz, const int* row_id, const int*
         int cap = 0;
         for (int b = 0; b < rows; b += per) cap = std::max(cap, ptr[(size_t)std::min(rows, b + per)] - ptr[(size_t)b]);
         if ((per <= kThreads || c == l.ctas) && per <= 0xffff && smem_of_rows(per, cap) <= l.smem && cap <= kEntriesPerCta) {
+            for (int b = 0; b < rows; b += per)
+                if (rows_step_us(ptr.get(), col, rows, per, b) > (row_id ? kCooStep : kCsrStep)) return p;
             p.ctas = c;
             p.per = per;
             p.cap = cap;

@@ -701,7 +701,8 @@ int clspmv_cocktail_set_csr_lanes(clspmv_cocktail_handle* h, int lanes);
  * Stream ordered with no host synchronisation (the reference waits after
  * every step): from 4 steps on, one DIA, BDIA, COO or CSR part whose rows fit
  * is held by the shared memory of one thread-block cluster and takes one
- * launch; otherwise whole groups of 16 steps replay one CUDA graph captured
+ * launch, unless its steps are estimated at upload to take longer that way
+ * (many diagonals, long rows, columns far from the diagonal); otherwise whole groups of 16 steps replay one CUDA graph captured
  * once per (x, y, alpha, beta) and cached in the handle, the rest launch
  * directly, and with beta = 0 on a square matrix the steps go back and forth
  * between x and y in place of the copies.

@@ -47,8 +47,11 @@ CASES = {"one": (lambda: _banded(1, 1, [0], 1), True, True), "grid6": (lambda: _
          "grid100": (lambda: _grid(100), True, True), "grid256": (lambda: _grid(256), True, True),
          "grid300": (lambda: _grid(300), False, False), "wide": (lambda: _banded(2500, 2600, [-70, -3, 0, 1, 2, 90, 99], 2, 0.8), True, True),
          "holes": (lambda: _banded(17000, 17000, [-5000, -2, 0, 3, 9000], 3, 0.7), True, True),
-         "uneven": (lambda: _uneven(9000, 9000, 12, 4), None, True), "long64": (lambda: _uneven(700, 900, 64, 5), None, True),
-         "long80": (lambda: _uneven(700, 700, 80, 6), None, False)}
+         "uneven": (lambda: _uneven(9000, 9000, 12, 4), None, False), "few": (lambda: _uneven(700, 760, 12, 5), None, True),
+         "long80": (lambda: _uneven(700, 700, 80, 6), None, False),
+         "near": (lambda: _banded(9000, 9000, np.arange(-7, 8), 8, 0.5), True, True),
+         "band40": (lambda: _banded(4000, 4000, np.arange(-20, 20), 9), None, False),
+         "band150": (lambda: _banded(900, 900, np.arange(-75, 75), 9), False, False)}
 
 
 @pytest.mark.parametrize("fmt", ["dia", "bdia", "coo", "csr"])
@@ -88,3 +91,37 @@ def test_every_entry_and_the_launches(fmt, name):
             assert torch.equal(x[:h], y) and torch.equal(x[h:], x0[h:])
             lim = 1.02 * k * (longest + 3) * 2.0 ** -24 * yd
             assert bool(((y.double() - yd).abs() <= lim).all()), (k, alpha, beta, float(((y.double() - yd).abs() / yd).max()))
+
+
+@pytest.mark.parametrize("fmt,name", [("coo", "uneven"), ("csr", "uneven"), ("coo", "band40"), ("csr", "band40"), ("bdia", "band150"),
+                                      ("bdia", "band40"), ("dia", "grid100"), ("csr", "grid256")])
+def test_no_slower_than_single_steps(fmt, name):
+    """A cluster that holds the matrix reads other CTAs' entries one after another: uneven rows took 3, bands 2 to 4 times
+    as long as the single steps."""
+    h, w, r, c = CASES[name][0]()
+    coo = F.coo_matrix(h, w, r, c, np.full(r.size, 1e-3, np.float32))
+    part = coo if fmt == "coo" else getattr(F, f"coo2{fmt}")(coo)
+    st = _abi.Cocktail()
+    st.mat_height, st.mat_width, st.mat_nnz = h, w, coo.nnz
+    setattr(st, f"ifuse{fmt}", True)
+    setattr(st, fmt, type(getattr(st, fmt)).from_buffer_copy(part.struct))
+    dev = CK.CocktailMatrix(st, owner=None).to_device()
+    x, y = torch.rand(w, device="cuda"), torch.rand(h, device="cuda")
+
+    def us(f):
+        times = []
+        for _ in range(9):
+            e = [torch.cuda.Event(enable_timing=True) for _ in range(2)]
+            e[0].record()
+            f()
+            e[1].record()
+            torch.cuda.synchronize()
+            times.append(e[0].elapsed_time(e[1]) * 1000)
+        return float(np.median(times[2:]))
+
+    g = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(g):
+        for _ in range(48):
+            dev.spmv(x, y, 1.0, 0.5)
+            x[:h].copy_(y)
+    assert us(lambda: dev.iterate(x, y, 48, 1.0, 0.5)) <= 1.25 * us(g.replay)
