@@ -1084,9 +1084,11 @@ template <class T, bool IS_CSR>
 int launch_chunks(int rows, int nnz, const int* row_ptr, const int* row_id, const int* col_id, const void* vals, Dense d,
                   int vec, cudaStream_t st)
 {
-    // 8 nonzeros per lane from where their runs fill the device's warps (1.2M nonzeros): 4 loses up to 1.4x there
-    // at k <= 16 (more searches and scans a nonzero) and wins 1.1-1.4x on 0.24M nonzeros (more warps)
-    const bool few = nnz < 148 * 32 * 256;
+    // 8 nonzeros per lane once their runs are a third more than the device's warps (1.6M nonzeros): 4 costs 5-10 % at
+    // k < 8 from there on (more searches and scans a nonzero); before, where most warps would take 2 runs of 8 and half of
+    // them none, it takes 1.2-1.4M nonzeros at k = 7 / 32 / 128 from 46 / 54 / 155 to 40 / 45 / 134 us (300,000 rows, 3 of 10
+    // filled), 28 / 36 / 83 to 25 / 29 / 65 (62,000 uneven rows)
+    const bool few = nnz < 148 * 32 * 256 / 3 * 4;
     // Few nonzeros leave warps idle while a slot of G lanes walks its 4 G nonzeros: G is halved, down to 4 lanes, until the
     // panels of G lanes' columns make 3/8 of the device's warps (all of them: 20,000 rows of 9 at k = 64 17 -> 19 us; down to 2
     // lanes: 3,000 rows of 4 at k = 12 15 -> 21). beta 0, us: 5,000 rows of 3 at k = 36 / 128 19 / 23 -> 13 / 13 (at beta 1
@@ -1096,10 +1098,13 @@ int launch_chunks(int rows, int nnz, const int* row_ptr, const int* row_id, cons
         while (lg > 2 && ((long long)nnz + 127) / 128 * ((d.k + (vec << lg) - 1) / (vec << lg)) < 148 * 12) lg--;
     // A CSR row is added, not written, where Y holds beta * Y already: a row that reads its Y first waits for it, one
     // row after another in a slot. beta = 1, us written / added: 5,000 rows of 3 at k = 36 27 / 14, 2^20 rows of 2 at
-    // k = 5 / 36 / 128 45 / 33, 157 / 125, 355 / 343. Other beta than 0 take a pass over Y for that, which pays for
-    // single columns (k < 8 or rows off 16 bytes) of a small Y: 200,000 rows of 9 at k = 5 47 / 35, 20,000 18 / 15,
-    // but 2^20 rows of 2 51 / 54, and at k = 16 60,000 rows 12.8 / 16.9.
-    const bool add = d.beta == 1.0f || (d.beta != 0.0f && vec == 1 && (long long)rows * d.k <= 1 << 20);
+    // k = 5 / 36 / 128 45 / 33, 157 / 125, 355 / 343. Other beta than 0 take a pass over Y for that, which pays for a
+    // small Y: up to 4 MB for single columns (k < 8 or rows off 16 bytes; 20,000 rows of 9 at k = 5 18 / 15 us) and, where
+    // rows hold 3 entries and more on average, 10 MB for those (300,000 rows of 4.5 at k = 7 53 / 48) and 4 MB for
+    // others (30,000 rows of 47 at k = 12 / 28 44 / 28, 58 / 43), but 60,000 rows of 2 at k = 16 12.8 / 16.9.
+    const long long floats = (long long)rows * d.k;
+    const bool filled = nnz >= 3LL * rows;
+    const bool add = d.beta == 1.0f || (d.beta != 0.0f && floats <= (vec == 1 && filled ? 5 << 19 : vec == 1 || filled ? 1 << 20 : 0));
     if (d.beta != 1.0f) {
         if (IS_CSR && nnz > 0 && !add)
             (vec == 4 ? k_scale_cut<4> : k_scale_cut<1>)<<<grid_of(rows), kSpmmBlock, 0, st>>>(

@@ -90,3 +90,26 @@ def test_few_nonzeros_take_more_warps():
     """5,000 rows of 3: k = 128 took 1.8 times as long as k = 16."""
     m = _device(5000, 1, 3)
     assert _us(m, 128, 0.0) <= 1.45 * _us(m, 16, 0.0)
+
+
+@pytest.mark.parametrize("h,per,k", [(30_000, 47, 12), (20_000, 9, 36), (60_000, 20, 5)])
+def test_beta_costs_no_more_than_a_pass_over_y(h, per, k):
+    """beta = 0.5 beside beta = 1 and a scaling of Y: rows that wait for their Y took up to 1.8 times as long."""
+    m = _device(h, 1, per)
+    Y = torch.rand((h, k), device="cuda")
+
+    def scaled():
+        Y.mul_(0.5)
+        m.spmm(X, Y, 0.5, 1.0)
+
+    X = torch.rand((h, k), device="cuda")
+    times = []
+    for _ in range(12):
+        a, b = (torch.cuda.Event(enable_timing=True) for _ in range(2))
+        a.record()
+        for _ in range(10):
+            scaled()
+        b.record()
+        torch.cuda.synchronize()
+        times.append(a.elapsed_time(b) * 100)
+    assert _us(m, k, 0.5) <= 1.2 * float(np.median(times[2:]))
