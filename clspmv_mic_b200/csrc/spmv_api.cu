@@ -1104,7 +1104,7 @@ struct clspmv_sell_plan {
     long long sector_bytes = 0;   // col + data bytes of the 32-byte sectors holding real entries
     long long line_bytes = 0;     // bytes the split walk must read in 128-byte lines (see clspmv_sell_plan_line_bytes)
     bool few = false;          // columns for fewer than a quarter of the device's warps' whole runs (sell_run)
-    int even = 0;              // little padding and at most this many columns on average (12 or 32), 0: else
+    int even = 0;              // little padding, at most this many columns on average (12 or 32) and twice that in any slice, 0: else
     bool split = true;         // walk the heads and the tails apart (power-of-two slice heights)
     bool compact = true;       // the tails' column ids from tail_col
 };
@@ -1197,8 +1197,11 @@ int clspmv_sell_plan_create(const clspmv_sell_f32* m, clspmv_sell_plan** out)
             for (uint64_t w : cline) lines += __builtin_popcountll(w);
             p->line_bytes = 128 * lines + 4 * tail_entries + 4 * rows + 4 * (ns + 1) + 12 * (long long)split.size() + 4;
             const long long slots = sp[(size_t)ns];
+            long long widest = 0;
+            for (long long q = 0; q < ns; q++) widest = std::max(widest, (long long)(sp[(size_t)q + 1] - sp[(size_t)q]) / shs);
             if (shs % 4 == 0 && ns * shs >= rows && 4 * p->line_bytes >= 3 * 8 * slots)
                 p->even = slots <= 12 * ns * shs ? 12 : slots <= 32 * ns * shs ? 32 : 0;
+            if (widest > 2 * p->even) p->even = 0;   // one thread walks a whole row: 300,000 entries took 65 ms (split walk 56 us)
         }
         // CLSPMV_SELL_SPLIT=0 walks every column instead, CLSPMV_SELL_TAIL_COMPACT=0
         // reads the tails' column ids in place (for measurements)
