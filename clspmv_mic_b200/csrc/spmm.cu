@@ -752,7 +752,7 @@ __global__ void __launch_bounds__(kSpmmBlock, 4) k_spmm_runs(int rows, int nnz, 
     static_assert(P % U == 0, "a batch of X rows stays within a lane's nonzeros");
     using XT = typename Acc<VEC>::X;
     const int lane = threadIdx.x & 31, slot = lane >> LG;
-    const int c0 = ((int)blockIdx.y * G + (lane & (G - 1))) * VEC;
+    const int c0 = ((P == 4 ? (int)blockIdx.y * G : 0) + (lane & (G - 1))) * VEC;   // panels only for few nonzeros (P = 4)
     const bool cols = c0 < d.k;
     const float* __restrict__ X = d.X + (cols ? c0 : 0);
     float* const Y = d.Y + c0;
