@@ -158,7 +158,7 @@ class DeviceCocktail:
         """`iterations` steps of y <- alpha * A x + beta * y; x[:rows] <- y
         (the reference's A^k x loop, src/eval.cpp:19-72), asynchronous on
         `stream`, in one launch where a single part fits a cluster's shared
-        memory, else replayed from a cached CUDA graph (clspmv_cocktail_iterate_f32)."""
+        memory and is faster there, else replayed from a cached CUDA graph (clspmv_cocktail_iterate_f32)."""
         from .formats import _stream_handle
         check(lib().clspmv_cocktail_iterate_f32(self.handle, x.data_ptr(), y.data_ptr(), alpha, beta, int(iterations),
                                                 _stream_handle(stream)), "cocktail_iterate")

@@ -20,7 +20,7 @@
 // (k_front) checks ids and order, builds the row pointer, and makes CSR's
 // copies or marks the diagonals on the way. Each padded layout is then
 // written once, every byte of it coalesced: ELL and SELL by quads of rows,
-// DIA by rows whose entries are staged in shared memory, and the 4-wide block
+// DIA by rows whose entries are staged in shared memory, whole or by windows, and the 4-wide block
 // formats by merging the sorted rows of a block row (k_blocks), without
 // sorting. Entries a row holds twice keep the last value in COO order, as in
 // the host loops. The generic BCSR / BELL of any block shape group their
@@ -1425,7 +1425,11 @@ template <int V> using ic = std::integral_constant<int, V>;
 template <class F>
 void with_shape(int bw, int bh, F&& f)
 {
-#define SHAPE(H)                                        if (bh == H) {                                          if (bw == 4) f(ic<H>{}, ic<4>{});                   else f(ic<H>{}, ic<8>{});                       }
+#define SHAPE(H)                      \
+    if (bh == H) {                    \
+        if (bw == 4) f(ic<H>{}, ic<4>{}); \
+        else f(ic<H>{}, ic<8>{});     \
+    }
     SHAPE(1)
     SHAPE(2)
     SHAPE(4)

@@ -235,8 +235,8 @@ Limits raised_limits()
     return l;
 }
 
-// CTAs of the cluster that holds the matrix, 0 if none does: as few as give
-// each one row per thread, more where the values need the room. A step took
+// Entries that a CTA holds at most. The cluster has as few CTAs as give each
+// one row per thread, more where the values need the room. A step took
 // 1.4 us with 1 row per thread and 2.7 with 4 (5 diagonals, 16 CTAs), against 4.0 for a
 // launch, and 4.1 with 6: past kEntriesPerCta the launches are the faster way.
 constexpr int kEntriesPerCta = 24 * 1024;

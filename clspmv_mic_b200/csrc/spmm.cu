@@ -283,9 +283,9 @@ __device__ __forceinline__ const int* cols_of(const clspmv_sell_f32& m) { return
 // 32 warps. The row walk has 4 a lane at 64 warps for FP32 ELL, which keeps
 // it, but fewer for 16-bit values and one for SELL, whose slot count the
 // compiler does not see; short rows keep it too. Slots are summed in the same order.
-// B200, 27-point stencil of 101^3, us at k = 8 / 16 / 64: SELL 187 / 341 /
-// 1222 -> 94 / 170 / 612, ELL with BF16 values 123 / 225 / 822 -> 92 / 166 /
-// 595; SELL of the power law of 2^20 rows at k = 8 7.2 -> 2.1 ms.
+// B200, 27-point stencil of 101^3, us at k = 8 / 16 / 64: SELL 184 / 329 /
+// 1180 -> 95 / 170 / 613, ELL with BF16 values 120 / 218 / 795 -> 92 / 166 /
+// 597; SELL of the power law of 2^20 rows at k = 8 7.2 -> 2.1 ms.
 constexpr int kSlotLoads = 8;
 template <int VEC, class T, class M>
 __global__ void __launch_bounds__(kSpmmBlock, 4) k_spmm_slots(M m, const T* __restrict__ vals, Dense d)
@@ -566,25 +566,26 @@ __global__ void __launch_bounds__(kSpmmBlock) k_spmm_warp_rows(int rows, const i
 // with 128-bit loads, finds the row of each (CSR: from row_ptr), and splits
 // its lanes into slots of G = 2^LG lanes that share the k columns of X and Y
 // (VEC columns a lane), or those of the block's panel (blockIdx.y) where few
-// nonzeros are worth more warps than that. A slot owns the P G nonzeros that its lanes loaded
-// and hands them round by shuffles, with kRunLoads X rows in flight: ids,
-// values and rows are read once, coalesced, and no lane waits for row_ptr
-// between two nonzeros.
+// nonzeros are worth more warps than that. A slot owns the P G nonzeros that
+// its lanes loaded and hands them round by shuffles, with kRunLoads X rows in
+// flight: ids, values and rows are read once, coalesced, and no lane waits for
+// row_ptr between two nonzeros.
 //
 // A CSR row that starts and ends in its warp's run is written directly
 // (alpha, beta), its pieces in several slots summed by a segmented scan, so
-// Y gets no scaling pass of its own (ADD: for beta = 1 it is added). Only rows cut by an edge between warps
+// Y gets no scaling pass of its own. Only rows cut by an edge between warps
 // are added atomically, after k_scale_cut has applied beta to those and to
-// the rows without entries. COO has no row pointer to tell them by: beta is
+// the rows without entries. With ADD (beta = 1, or Y scaled before) every row
+// is added: a row that reads its Y would wait for it. COO has no row pointer to tell them by: beta is
 // applied to all of Y first and every row is added, by red.global.add, which
 // a slot does not wait for.
 //
 // Measured on B200 (us, CSR, FP32; before: 16 nonzeros per lane group, a
 // search of row_ptr for each, Y zeroed first and every row read, added and
-// written): power law of 2^20 rows, k = 4 / 16 / 32: 186 / 325 / 566 -> 105 /
-// 197 / 345; 27-point stencil of 100^3: 266 / 376 / 621 -> 127 / 250 / 432.
+// written): power law of 2^20 rows, k = 4 / 16 / 32: 187 / 327 / 568 -> 103 /
+// 198 / 344; 27-point stencil of 100^3: 268 / 378 / 623 -> 122 / 253 / 424.
 // At k = 16 on the power law it moves its 1.04 GB of X rows at 5.3 TB/s (X is
-// 64 MB: L2 hits 57 %), at k = 64 at 6.4 TB/s, the rate of DRAM. Also measured, not
+// 64 MB: L2 hits 58 %), at k = 64 DRAM carries 3.5 GB at 0.87 of the copy rate. Also measured, not
 // kept: rows walked within equal ranges of nonzeros, several slots a row
 // (358 us at k = 16 on the power law), ends of rows written without a branch
 // (280), evict-last X or streaming Y (within 3 %), 3 CTAs per SM (198).
@@ -1058,7 +1059,7 @@ int launch_blocks(const M& m, const void* vals, Dense d, int vec, cudaStream_t s
     return after_launch(1);
 }
 
-// CLSPMV_SPMM_WARP_ROWS=0 keeps the nonzero-chunk kernel for long CSR rows (measurements).
+// CLSPMV_SPMM_WARP_ROWS=0 takes long CSR rows by warp runs too (measurements).
 bool warp_rows_enabled()
 {
     static const bool on = [] {

@@ -1252,9 +1252,9 @@ int launch_sell_even(const clspmv_sell_f32* m, const V* data, const float* scale
 }
 // Nearly every line holds entries (on the power law 0.6 of them) and rows are
 // short: nothing for the split walk to save, and 4 rows per thread need no
-// scaled y, no atomics and no shuffles. Measured on B200 (us, split walk -> 4
-// rows per thread): 5-point Laplacian of 2k / 200k / 1M rows 30 / 28 / 41 ->
-// 3.6 / 4.6 / 10.5, rows of 9 with BF16 values at 1M 39 -> 21; 1M rows of 27
+// scaled y, no atomics and no shuffles. Measured on B200 (us of a call, split
+// walk -> 4 rows per thread): 5-point Laplacian of 2k / 4k / 200k / 1M rows 31 /
+// 33 / 35 / 52 -> 6 / 6 / 6.5 / 12.7, rows of 9 with BF16 values at 1M 39 -> 21; 1M rows of 27
 // 64 -> 56, of 10 to 30 at random 117 -> 99. Rows of 13 to 32 in smaller matrices leave
 // the thread's walk too few threads (2k rows of 31: 10.2 us against 6.8 for
 // runs of columns), and with 16-bit values it is the slower one (1M of 27: 53 -> 62).

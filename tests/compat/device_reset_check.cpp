@@ -17,11 +17,11 @@ static F fn(const char* name) { return reinterpret_cast<F>(dlsym(so, name)); }
 
 static int failures = 0;
 #define CHECK(c) \
-    do { if (!(c)) { failures++; printf("round %d, line %d: %s\n", round, __LINE__, #c); } } while (0)
+    do { if (!(c)) { failures++; printf("pass %d, line %d: %s\n", pass, __LINE__, #c); } } while (0)
 
 static constexpr int N = 16000;   // a cluster of 16 blocks, more than a kernel may have by default
 
-static void upload(int round)   // twice the identity, its arrays over 2 MB so that they have pages of their own
+static void upload(int pass)   // twice the identity, its arrays over 2 MB so that they have pages of their own
 {
     const int n = 1 << 20;
     std::vector<int> rp(n + 1), col(n);
@@ -34,7 +34,7 @@ static void upload(int round)   // twice the identity, its arrays over 2 MB so t
     h.csr_col_id = col.data();
     h.csr_data = val.data();
     float *dx = nullptr, *dy = nullptr, *mine[4];
-    for (float*& p : mine) {   // the caller's own, which may lie where the last round's arrays lay
+    for (float*& p : mine) {   // the caller's own, which may lie where the last pass's arrays lay
         CHECK(cudaMalloc(&p, 4 * n) == cudaSuccess);
         CHECK(cudaMemcpy(p, x.data(), 4 * n, cudaMemcpyHostToDevice) == cudaSuccess);
     }
@@ -53,7 +53,7 @@ static void upload(int round)   // twice the identity, its arrays over 2 MB so t
     CHECK(fn<decltype(&clspmv_device_free_csr_f32)>("clspmv_device_free_csr_f32")(&d) == CLSPMV_OK);
 }
 
-static void iterate(int round)   // 8 steps of x <- A x, A the permutation that shifts by one row
+static void iterate(int pass)   // 8 steps of x <- A x, A the permutation that shifts by one row
 {
     int off = 1;
     const int len = (N + 31) / 32 * 32;
@@ -92,9 +92,9 @@ static void iterate(int round)   // 8 steps of x <- A x, A the permutation that 
 int main(int argc, char** argv)
 {
     if (argc < 3 || !(so = dlopen(argv[1], RTLD_NOW))) return 99;
-    for (int round = 0; round < 3; round++) {
-        if (std::string(argv[2]) == "iterate") iterate(round);
-        else upload(round);
+    for (int pass = 0; pass < 3; pass++) {
+        if (std::string(argv[2]) == "iterate") iterate(pass);
+        else upload(pass);
         if (failures) break;
         CHECK(cudaDeviceReset() == cudaSuccess);
     }
