@@ -37,18 +37,24 @@ def _device(h, filled, per):
     return F.device_convert(F.DeviceMatrix.from_device_arrays("coo", dict(width=h, height=h, nnz=col.numel()), coo), "csr")
 
 
-def _us(m, k, beta):
-    X, Y = (torch.rand((m.shape[0], k), device="cuda") for _ in range(2))
+def _median_us(f):
+    for _ in range(50):   # clocks and caches as in a stream of calls
+        f()
     times = []
-    for _ in range(12):
+    for _ in range(21):
         a, b = (torch.cuda.Event(enable_timing=True) for _ in range(2))
         a.record()
         for _ in range(10):
-            m.spmm(X, Y, 0.5, beta)
+            f()
         b.record()
         torch.cuda.synchronize()
         times.append(a.elapsed_time(b) * 100)
-    return float(np.median(times[2:]))
+    return float(np.median(times))
+
+
+def _us(m, k, beta):
+    X, Y = (torch.rand((m.shape[0], k), device="cuda") for _ in range(2))
+    return _median_us(lambda: m.spmm(X, Y, 0.5, beta))
 
 
 @pytest.mark.parametrize("h,filled,per", [(1, 1, 1), (31, 0.5, 3), (257, 0.1, 9), (3001, 0.02, 40), (5000, 1, 2), (700, 0.5, 31)])
@@ -89,7 +95,8 @@ def test_rows_do_not_wait_for_their_y():
 def test_few_nonzeros_take_more_warps():
     """5,000 rows of 3: k = 128 took 1.8 times as long as k = 16."""
     m = _device(5000, 1, 3)
-    assert _us(m, 128, 0.0) <= 1.45 * _us(m, 16, 0.0)
+    first, second = ([_us(m, k, 0.0) for k in (128, 16)] for _ in range(2))   # of calls this short the best of two
+    assert min(first[0], second[0]) <= 1.45 * min(first[1], second[1])
 
 
 @pytest.mark.parametrize("h,per,k", [(30_000, 47, 12), (20_000, 9, 36), (60_000, 20, 5)])
@@ -103,13 +110,4 @@ def test_beta_costs_no_more_than_a_pass_over_y(h, per, k):
         m.spmm(X, Y, 0.5, 1.0)
 
     X = torch.rand((h, k), device="cuda")
-    times = []
-    for _ in range(12):
-        a, b = (torch.cuda.Event(enable_timing=True) for _ in range(2))
-        a.record()
-        for _ in range(10):
-            scaled()
-        b.record()
-        torch.cuda.synchronize()
-        times.append(a.elapsed_time(b) * 100)
-    assert _us(m, k, 0.5) <= 1.2 * float(np.median(times[2:]))
+    assert _us(m, k, 0.5) <= 1.2 * _median_us(scaled)
